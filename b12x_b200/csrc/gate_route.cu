@@ -3,16 +3,17 @@
 //
 //   gate_route_simt_kernel  any operand types (bf16 / f32), any K, E <= 1024.  A CTA multiplies
 //       4 tokens x 32 experts on the CUDA cores; the last CTA of a token group to finish (a
-//       counter per group, no waiting) routes that group's tokens.  Decode batches: the grid
-//       spreads the gate matrix over many SMs.
-//   gate_route_tc_kernel    bf16 x bf16, E a multiple of 16 and <= 256.  One CTA per 128 tokens:
-//       TMA-fed tcgen05.mma (kind::f16) with the E logits of a token in one TMEM lane; the epilogue
-//       writes the logits and routes its 32 tokens per warp.  Prefill batches.
+//       counter per group, no waiting) routes that group's tokens.
+//   gate_route_tc_kernel    bf16 x bf16, E a multiple of 16 and <= 256.  A cluster of one to eight
+//       CTAs per 128 tokens: TMA-fed tcgen05.mma (kind::f16) with the E logits of a token in one
+//       TMEM lane, each CTA over its part of K; the parts are summed through distributed shared
+//       memory and the tokens routed by the warp that sums them.
 //
 // The logits are produced as the reference does (b12x/moe/fused_moe/_impl.py:11461-11468: a matrix
 // product written in the operands' common type, then the bias added in that type): fp32
 // accumulation, one rounding to bf16 when both operands are bf16, the bias added with one more
 // rounding.  The router then works on the stored logits (same routine as b200moe_route_topk).
+#include "cluster_pair.cuh"
 #include "gemm_shared.cuh"
 #include "route_shared.cuh"
 
@@ -54,16 +55,12 @@ __device__ __forceinline__ float finish_logit(float acc, const void* bias, int e
   return v;
 }
 
-template <int MODE>
-__device__ __forceinline__ void route_rows(const b200moe_route_args& r, int t0, int n, int warp_in_group,
-                                           int warps_in_group, int lane) {
-  for (int i = warp_in_group; i < n; i += warps_in_group) route_topk_token<MODE, true>(r, t0 + i, lane);
-}
-
-__device__ __forceinline__ void route_rows_any(const b200moe_route_args& r, int t0, int n, int wig, int nw, int lane) {
-  if (r.mode == B200MOE_ROUTE_SOFTMAX_TOPK) route_rows<B200MOE_ROUTE_SOFTMAX_TOPK>(r, t0, n, wig, nw, lane);
-  else if (r.mode == B200MOE_ROUTE_RAW) route_rows<B200MOE_ROUTE_RAW>(r, t0, n, wig, nw, lane);
-  else route_rows<B200MOE_ROUTE_SIGMOID>(r, t0, n, wig, nw, lane);
+// one warp routes token t
+template <int PER>
+__device__ __forceinline__ void route_token_any(const b200moe_route_args& r, int t, int lane) {
+  if (r.mode == B200MOE_ROUTE_SOFTMAX_TOPK) route_topk_token<B200MOE_ROUTE_SOFTMAX_TOPK, PER, true>(r, t, lane);
+  else if (r.mode == B200MOE_ROUTE_RAW) route_topk_token<B200MOE_ROUTE_RAW, PER, true>(r, t, lane);
+  else route_topk_token<B200MOE_ROUTE_SIGMOID, PER, true>(r, t, lane);
 }
 
 __global__ void __launch_bounds__(256) gate_route_simt_kernel(b200moe_gate_route_args g, b200moe_route_args r,
@@ -148,12 +145,24 @@ __global__ void __launch_bounds__(256) gate_route_simt_kernel(b200moe_gate_route
   if (!is_last) return;
   __threadfence();
   const int n = min(kGateTok, T - t0);
-  if (warp < n) route_rows_any(r, t0, n, warp, 8, lane);
+  if (warp < n) {
+    if (E <= 256) route_token_any<8>(r, t0 + warp, lane);
+    else route_token_any<32>(r, t0 + warp, lane);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
-constexpr int kTcThreads = 192;       // TMA warp, MMA warp, four epilogue warps
+// Split over the reduction.  A 128-token tile has to see the whole gate matrix (E x K x 2 bytes:
+// 3.7 MB at 256 x 7168, which one SM takes some 35 us to bring in from L2), and a batch has few
+// tiles, so a CLUSTER of up to eight CTAs shares one: each multiplies its part of K into its own
+// TMEM accumulator, leaves the fp32 partial sums in shared memory, and after a cluster barrier
+// sums the parts of 128 / S of the tokens out of the S shared memories, in order of S, rounds
+// them and routes those tokens, one warp per token.  4096 tokens x 256 experts, K 7168: 332 us with
+// one CTA per tile (32 SMs, each of four warps routing 32 tokens), 40 us now (28 us with the
+// operands in L2); what is left is the operands' way into each SM and the routing at the end.
+constexpr int kTcThreads = 512;       // TMA warp, MMA warp, four epilogue warps; all sixteen warps route
 constexpr int kTcStages = 4;
+constexpr int kTcMaxSplit = 8;        // portable cluster size
 struct __align__(8) GateTail {
   uint64_t full[kTcStages];
   uint64_t empty[kTcStages];
@@ -162,9 +171,15 @@ struct __align__(8) GateTail {
   int abort_flag;
 };
 
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 __global__ void __launch_bounds__(kTcThreads, 1)
 gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-                     b200moe_gate_route_args g, b200moe_route_args r, int tmem_cols) {
+                     b200moe_gate_route_args g, b200moe_route_args r, int tmem_cols, int splits) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -174,8 +189,14 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   uint8_t* sW = sX + kTcStages * 16384;              // [stage][E rows][128 bytes]
   GateTail* tail = reinterpret_cast<GateTail*>(sW + kTcStages * ((smem_w + 1023) & ~1023));
   const int w_stage = (smem_w + 1023) & ~1023;
+  // the partial sums of this CTA take the place of the stages once its MMAs are done: 128 rows of
+  // E + 4 floats (the pad spreads the rows a warp writes over the banks), 512 E + 2048 bytes
+  float* sPart = reinterpret_cast<float*>(smem);
+  const int part_stride = E + 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_blocks = (K + 63) / 64;                // 64 bf16 = one 128-byte swizzled row
+  const int rank = static_cast<int>(pair::cluster_ctarank());
+  const int kb0 = k_blocks * rank / splits, kb1 = k_blocks * (rank + 1) / splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTcStages; ++s) {
@@ -195,7 +216,7 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = tail->tmem_base;
   volatile int* abort_flag = &tail->abort_flag;
-  const int t0 = blockIdx.x * 128;
+  const int t0 = static_cast<int>(blockIdx.x) / splits * 128;
 
   if (warp == 0) {
     if (lane < 2) {
@@ -206,7 +227,7 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait_bounded(&tail->empty[stage], phase ^ 1, abort_flag, g.status, WAIT_SMEM_EMPTY)) {
           ok = false;
           break;
@@ -233,7 +254,7 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait_bounded(&tail->full[stage], phase, abort_flag, g.status, WAIT_SMEM_FULL)) {
           ok = false;
           break;
@@ -244,7 +265,7 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         // four MMAs of 16 elements; the zero-filled tail of the last k-block adds nothing
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          mma_bf16(tmem_base, adesc + 2 * j, bdesc + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+          mma_bf16(tmem_base, adesc + 2 * j, bdesc + 2 * j, idesc, (kb > kb0 || j > 0) ? 1u : 0u);
         tc_commit(&tail->empty[stage]);
         if (++stage == kTcStages) {
           stage = 0;
@@ -253,45 +274,60 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       }
       if (ok) tc_commit(&tail->acc_full);
     }
-  } else {
-    // epilogue: warp w reads TMEM sub-partition w & 3 = tokens t0 + 32 * (w & 3) + lane
+  } else if (warp >= 4 && warp < 8) {
+    // epilogue: warp w reads TMEM sub-partition w & 3 = tokens t0 + 32 * (w & 3) + lane.  acc_full
+    // says that every MMA has read its stage, so the partial sums may overwrite the stages.
     const int sub = warp & 3;
-    const int t = t0 + sub * 32 + lane;
     if (mbar_wait_bounded(&tail->acc_full, 0, abort_flag, g.status, WAIT_TMEM_FULL)) {
       tc_fence_after();
       const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(sub * 32) << 16);
-      __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(g.logits_out) + static_cast<int64_t>(t) * E;
+      float* row = sPart + (sub * 32 + lane) * part_stride;
       for (int c = 0; c < E; c += 16) {
         uint32_t v[16];
         tc_ld_32x32b_x16(t_lane + c, v);
         tc_wait_ld();
-        if (t < T) {
-          uint32_t pk[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float a = finish_logit(__uint_as_float(v[2 * i]), g.gate_bias, c + 2 * i, g.bias_dtype, true);
-            const float b = finish_logit(__uint_as_float(v[2 * i + 1]), g.gate_bias, c + 2 * i + 1, g.bias_dtype, true);
-            pk[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a))) |
-                    (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(b))) << 16);
-          }
-          uint4* dst = reinterpret_cast<uint4*>(row + c);
-          dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        }
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(row + c + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
       }
-      // this warp's 32 rows are in global memory: route them
-      __threadfence();
-      __syncwarp();
-      const int n = min(32, T - (t0 + sub * 32));
-      if (n > 0) route_rows_any(r, t0 + sub * 32, n, 0, 1, lane);
     }
   }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  pair::cluster_sync_all();      // every part of the tile is in shared memory
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, static_cast<uint32_t>(tmem_cols));
   }
+  // this CTA's share of the tile's tokens, one warp per token
+  const int share = 128 / splits;
+  const uint32_t part_addr = smem_u32(sPart);
+  for (int i = warp; i < share; i += kTcThreads / 32) {
+    const int row = rank * share + i;
+    const int t = t0 + row;
+    if (t >= T) break;
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+    for (int s = 0; s < splits; ++s) {
+      const uint32_t src = pair::map_to_cta(part_addr, static_cast<uint32_t>(s)) +
+                           static_cast<uint32_t>(row * part_stride) * 4u;
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = j * 32 + lane < E ? ld_cluster_f32(src + (j * 32 + lane) * 4) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], v[j]);
+    }
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.logits_out) + static_cast<int64_t>(t) * E;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int e = j * 32 + lane;
+      if (e < E) out[e] = __float2bfloat16_rn(finish_logit(acc[j], g.gate_bias, e, g.bias_dtype, true));
+    }
+    __syncwarp();                // the row is in global memory for the lane that reads the winner's logit
+    route_token_any<8>(r, t, lane);
+  }
+  pair::cluster_sync_all();      // nobody reads this CTA's shared memory after this
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -356,7 +392,12 @@ extern "C" int b200moe_gate_route(const b200moe_gate_route_args* g, void* stream
                      g->hidden_row_stride % 8 == 0 && aligned16(g->hidden) && aligned16(g->gate_weight) &&
                      aligned16(g->logits_out);
   int kernel = g->kernel;
-  if (kernel == B200MOE_GATE_AUTO) kernel = (tc_ok && T >= 128) ? B200MOE_GATE_TC : B200MOE_GATE_SIMT;
+  // The tensor-core kernel wherever its layout rules hold, down to one token (the CUDA-core kernel
+  // has E / 32 CTAs for a decode batch, each with 32 whole rows of the gate matrix to read):
+  // 256 x 7168 at 1 / 64 tokens 43 -> 13 / 51 -> 17 us, 64 x 512 10.2 -> 6.6 / 10.4 -> 8.0 us.  Below
+  // 32768 gate weights a decode batch stays on the CUDA cores (16 x 256 at 64 tokens: 8.2 against 9.5).
+  if (kernel == B200MOE_GATE_AUTO)
+    kernel = (tc_ok && (T >= 128 || static_cast<int64_t>(E) * K >= 32768)) ? B200MOE_GATE_TC : B200MOE_GATE_SIMT;
   if (kernel == B200MOE_GATE_TC) {
     if (!tc_ok) return B200MOE_EUNSUPPORTED;
     CUtensorMap tmX, tmW;
@@ -371,8 +412,24 @@ extern "C" int b200moe_gate_route(const b200moe_gate_route_args* g, void* stream
     const int smem = 1024 + kTcStages * (16384 + ((E * 128 + 1023) & ~1023)) + static_cast<int>(sizeof(GateTail));
     if (cudaFuncSetAttribute(gate_route_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return B200MOE_ECUDA;
-    gate_route_tc_kernel<<<(T + 127) / 128, kTcThreads, smem, s>>>(tmX, tmW, *g, r, cols);
-    return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
+    // as many parts of the reduction per token tile as keep all SMs busy, each with a k-block or more
+    const int tiles = (T + 127) / 128, k_blocks = (K + 63) / 64, sms = num_sms_cached();
+    int splits = kTcMaxSplit;
+    while (splits > 1 && (tiles * splits > sms || splits > k_blocks)) splits >>= 1;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(splits);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, gate_route_tc_kernel, tmX, tmW, *g, r, cols, splits) == cudaSuccess
+               ? B200MOE_OK : B200MOE_ECUDA;
   }
   if (kernel != B200MOE_GATE_SIMT) return B200MOE_EINVAL;
   const size_t he = g->hidden_dtype == B200MOE_DT_BF16 ? 2 : 4, we = g->weight_dtype == B200MOE_DT_BF16 ? 2 : 4;

@@ -5,11 +5,22 @@
 
 namespace b200moe {
 
-template <int MODE>
+template <int MODE, int PER>
 __global__ void __launch_bounds__(128) route_topk_kernel(b200moe_route_args a) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp >= a.num_tokens) return;
-  route_topk_token<MODE>(a, warp, threadIdx.x & 31);
+  route_topk_token<MODE, PER>(a, warp, threadIdx.x & 31);
+}
+
+template <int MODE>
+static void launch_route_topk(const b200moe_route_args& a, dim3 grid, cudaStream_t s) {
+  const int per_lane = (a.num_experts + 31) >> 5;     // values per lane, rounded up to a power of two
+  if (per_lane <= 1) route_topk_kernel<MODE, 1><<<grid, 128, 0, s>>>(a);
+  else if (per_lane <= 2) route_topk_kernel<MODE, 2><<<grid, 128, 0, s>>>(a);
+  else if (per_lane <= 4) route_topk_kernel<MODE, 4><<<grid, 128, 0, s>>>(a);
+  else if (per_lane <= 8) route_topk_kernel<MODE, 8><<<grid, 128, 0, s>>>(a);
+  else if (per_lane <= 16) route_topk_kernel<MODE, 16><<<grid, 128, 0, s>>>(a);
+  else route_topk_kernel<MODE, 32><<<grid, 128, 0, s>>>(a);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -370,13 +381,13 @@ extern "C" int b200moe_route_topk(const b200moe_route_args* a, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (a->mode) {
     case B200MOE_ROUTE_SOFTMAX_TOPK:
-      route_topk_kernel<B200MOE_ROUTE_SOFTMAX_TOPK><<<grid, 128, 0, s>>>(*a);
+      launch_route_topk<B200MOE_ROUTE_SOFTMAX_TOPK>(*a, grid, s);
       break;
     case B200MOE_ROUTE_RAW:
-      route_topk_kernel<B200MOE_ROUTE_RAW><<<grid, 128, 0, s>>>(*a);
+      launch_route_topk<B200MOE_ROUTE_RAW>(*a, grid, s);
       break;
     case B200MOE_ROUTE_SIGMOID:
-      route_topk_kernel<B200MOE_ROUTE_SIGMOID><<<grid, 128, 0, s>>>(*a);
+      launch_route_topk<B200MOE_ROUTE_SIGMOID>(*a, grid, s);
       break;
     default:
       return B200MOE_EINVAL;
