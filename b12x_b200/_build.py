@@ -21,7 +21,7 @@ SOURCES = (
     "grouped_gemm_bs.cu",
     "grouped_gemm_small.cu",
     "grouped_gemm_pair.cu",
-    "grouped_gemm_other.cu",
+    "grouped_gemm_w4a16.cu",
     "ep_peer.cu",
 )
 NVCC_FLAGS = (

@@ -157,6 +157,33 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same for a role that waits most of the time and is not in a hurry (a producer with a deep ring in
+// front of it, an epilogue with a second accumulator): it sleeps between two looks.  A warp that polls
+// takes issue slots from the warps that work beside it on its scheduler.
+__device__ __forceinline__ bool mbar_wait_idle(uint64_t* bar, uint32_t parity, volatile int* cta_abort, int* status,
+                                               int site) {
+  if (mbar_try_wait(bar, parity)) return true;
+  unsigned long long t0 = 0;
+  uint32_t spins = 0;
+  while (true) {
+    __nanosleep(100);
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((++spins & 0x3ffu) == 0) {
+      if (*cta_abort) return false;
+      const unsigned long long now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kWaitLimitNs) {
+        *cta_abort = 1;
+        if (status != nullptr) {
+          atomicCAS(status, 0, 1);
+          atomicCAS(status + 1, 0, site);
+        }
+        return false;
+      }
+    }
+  }
+}
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -115,7 +115,7 @@ class PeerExpertParallelMoE(_LayerBase):
         self.fold_waits = os.environ.get("B200MOE_FOLD_WAITS", "1") == "1"
         # route, home sort, dispatch, expert sort, file / quantise rows, FC1, FC2, combine (+ wait, signal, wait)
         self.kernels_per_step = (4 + sort_launches(t * k) + sort_launches(slots) + (0 if self.fold_waits else 3)
-                                 + gemm_launches(slots, self.n_local)
+                                 + gemm_launches(slots, self.n_local, shp.recipe)
                                  + (1 if self.replicas is not None else 0))
         # what crosses the link per route: the row quantised on this rank (the recipe's activation
         # format) or, for recipes whose GEMM reads bf16 rows, the row as it is

@@ -1,0 +1,70 @@
+"""-m gpu: the W4A16 kernels at the edges of their token tiles (16-column steps on one CTA, at most 64; 32-column
+steps on a CTA pair, at most 160), of their stages (two and four k-blocks of 64) and of their weight tiles, and the
+per-row power-of-two scaling of the FP16 token rows over the range of BF16."""
+
+from dataclasses import replace
+
+import pytest
+import torch
+
+from b12x_b200 import synth
+from tests.gpu_utils import oracle_layer, run_layer
+from tests.test_gpu_parity import _check_w4a16_layer, _w16
+
+pytestmark = pytest.mark.gpu
+
+
+def _one_expert(tokens, experts, hidden, inter, act="silu"):
+    """Every token on one expert of ``experts``: the plan's average decides the kernel, the expert's rows the tiles."""
+    shp = _w16(tokens=tokens, experts=experts, topk=1, hidden=hidden, intermediate=inter, activation=act)
+    ids = torch.full((tokens, 1), experts // 2, dtype=torch.int32)
+    return synth.make_inputs(shp, seed=tokens + hidden), ids, torch.full((tokens, 1), 0.75)
+
+
+@pytest.mark.parametrize("tokens", [1, 15, 16, 17, 32, 33, 63, 64, 65, 127, 130])
+@pytest.mark.parametrize("hidden,inter", [(64, 64), (320, 192)])      # one k-block; five and three
+def test_single_cta_token_tiles(tokens, hidden, inter):
+    inp, ids, w = _one_expert(tokens, 16, hidden, inter)
+    _check_w4a16_layer(run_layer(inp, topk_ids=ids, topk_weights=w))
+
+
+@pytest.mark.parametrize("tokens", [32, 33, 160, 161, 320, 321, 500])
+@pytest.mark.parametrize("hidden,inter,act", [(64, 64, "silu"), (448, 320, "silu"), (192, 192, "relu2")])
+def test_cta_pair_token_tiles(tokens, hidden, inter, act):
+    inp, ids, w = _one_expert(tokens, 1, hidden, inter, act)
+    _check_w4a16_layer(run_layer(inp, topk_ids=ids, topk_weights=w))
+
+
+def test_more_work_items_than_a_cta_lists_ahead():
+    """1024 experts x 40 weight tiles: more than 256 items on each of 148 SMs."""
+    shp = _w16(tokens=1024, experts=1024, topk=1, hidden=64, intermediate=2560)
+    ids = torch.randperm(1024, generator=torch.Generator().manual_seed(1)).to(torch.int32).reshape(-1, 1)
+    _check_w4a16_layer(run_layer(synth.make_inputs(shp, seed=3), topk_ids=ids, topk_weights=torch.ones(1024, 1)))
+
+
+def test_row_scaling_over_the_bf16_range():
+    shp = _w16(tokens=48, experts=2, topk=1, hidden=256, intermediate=128)
+    inp = synth.make_inputs(shp, seed=8)
+    gen = torch.Generator().manual_seed(9)
+    x = inp.x.float()
+    x[8:16] *= 2.0 ** 50
+    x[16:24] *= 2.0 ** -40
+    x[24:32] *= torch.exp2(torch.randint(-24, 1, (8, 256), generator=gen).float())   # a row over 24 binades
+    x[32] = 0.0
+    x[33, 1:] = 0.0
+    inp = replace(inp, x=x.to(torch.bfloat16))
+    ids = (torch.arange(48) % 2).to(torch.int32).reshape(-1, 1)
+    w = torch.ones(48, 1)
+    run = run_layer(inp, topk_ids=ids, topk_weights=w)
+    _, taps = oracle_layer(inp, ids, w)
+    # row by row, since their sizes lie 2^180 apart: 1e-2 x the row's RMS
+    err = (run.out_f32 - taps.out_f32).abs().amax(dim=1)
+    rms = taps.out_f32.double().square().mean(dim=1).sqrt().float()
+    assert bool((err <= 1e-2 * rms).all()), (err / rms.clamp(min=1e-38)).max()
+    # an infinity or a NaN stays in its own row
+    bad = x.clone()
+    bad[5, 7], bad[40, 3] = float("inf"), float("nan")
+    again = run_layer(replace(inp, x=bad.to(torch.bfloat16)), topk_ids=ids, topk_weights=w)
+    keep = [i for i in range(48) if i not in (5, 40)]
+    assert torch.equal(again.out_f32[keep], run.out_f32[keep])
+    assert not bool(torch.isfinite(again.out_f32[5]).any()) and bool(torch.isnan(again.out_f32[40]).all())
