@@ -35,6 +35,12 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
+// True in one lane of the (converged) warp.  Roles that one thread runs -- MMA issue, TMA producers --
+// are `if (elect_one())` regions and not `if (lane == 0)`: only from elect.sync does the compiler know
+// that a single thread is active, and without that every tcgen05.mma, tcgen05.commit and TMA copy pays
+// 40 to 60 clocks to bring its operands into uniform registers (four MMAs and two commits: 270 clocks
+// against 40).  On the layers: nvfp4 FC1 of the Mixtral shape at 8192 tokens 935 -> 847 us, decode of the
+// DeepSeek-V3 shape at 64 tokens 853 -> 811 us, w4a8_mx decode at 32 tokens 298 -> 260 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -279,7 +285,8 @@ __device__ __forceinline__ void tc_wait_st() {
 // Scale atoms (512 bytes each, `natoms` of them back to back in shared memory) -> `4 * natoms`
 // TMEM columns of this warp's sub-partition, atom j at columns [col_stride * j, +4): lane i takes
 // the 16 bytes of atom row i, as tcgen05.cp.32x128b.warpx4 would place them.  Called by one warp
-// per sub-partition; the tensor pipe is not involved.
+// per sub-partition; the tensor pipe is not involved.  (One 8- or 16-column store for two or four atoms
+// is slower, FC1 of the pair kernel 809 -> 877 / 947 us on 16 384 nvfp4 rows of the Mixtral shape.)
 template <int NATOMS>
 __device__ __forceinline__ void sf_atoms_to_tmem(uint32_t taddr, const uint8_t* atoms, int lane, int col_stride) {
 #pragma unroll

@@ -249,7 +249,7 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(128, E);
       int stage = 0;
       uint32_t phase = 0;

@@ -119,75 +119,57 @@ grouped_gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA,
   regs_release_to<kRegsSmall>();
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    // A few lanes walk the same loop and each issues ONE of the stage's copies: lane 0 arms the
-    // barrier and fetches A, lanes 1..kBoxes fetch the 64-row weight boxes, then one lane for the
-    // activation scale atoms and one per weight scale chain.
+    // One elected thread issues all copies of a stage.  (One lane per copy, as this was before, makes
+    // every copy an instruction of a divergent lane: tens of clocks each instead of a few.)
     constexpr int kBoxes = BN / 64;
-    constexpr int kLanes = 2 + kBoxes + Cfg::kSfbChains;
-    if (lane < kLanes) {
-      if (lane == 0) {
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmA_small);
-        tma_prefetch_desc(&tmB);
-      }
+    if (elect_one()) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmA_small);
+      tma_prefetch_desc(&tmB);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       TL_DECL(tl_n);
-      // Where this lane's copy of tile `w` comes from.  Tiles of a decode batch hold a few rows:
-      // they fetch 32 activation rows instead of 128 (the other rows of the shared-memory tile
-      // keep stale data; MMA rows are independent).  A gated tile is BN/128 pair groups: box 2g =
-      // 64 up rows, box 2g+1 = the 64 gate rows of the same columns; its scale chain g is the pair
-      // atom of those columns.  A plain tile is BN consecutive rows.
-      struct LaneSrc {
-        const CUtensorMap* tm;   // operand lanes
-        int y;                   // row coordinate
-        const uint8_t* sf;       // scale lanes: atom chain
-        uint32_t a_bytes;
-      };
-      auto locate = [&](int w) {
+      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+        // Tiles of a decode batch hold a few rows: they fetch 32 activation rows instead of 128 (the
+        // other rows of the shared-memory tile keep stale data; MMA rows are independent).  A gated
+        // tile is BN/128 pair groups: box 2g = 64 up rows, box 2g+1 = the 64 gate rows of the same
+        // columns; its scale chain g is the pair atom of those columns.  A plain tile is BN
+        // consecutive rows.
         const TileCoord c = decode_work(w, p, tail->tile_base);
-        LaneSrc r;
         const bool small_a = p.mtile_rows[c.mt] <= 32;
-        r.a_bytes = (small_a ? 32u : 128u) * kRowBytes;
-        r.tm = &tmB;
-        r.y = 0;
-        r.sf = p.sfa + static_cast<size_t>(c.mt) * p.atoms_k * 512;
-        if (lane == 0) {
-          r.tm = small_a ? &tmA_small : &tmA;
-          r.y = p.mtile_row0[c.mt];
-        } else if (lane <= kBoxes) {
-          const int b = lane - 1;
-          int my_row;
+        const uint32_t a_bytes = (small_a ? 32u : 128u) * kRowBytes;
+        const CUtensorMap* tma_a = small_a ? &tmA_small : &tmA;
+        const int row0 = p.mtile_row0[c.mt];
+        int y[kBoxes];
+#pragma unroll
+        for (int b = 0; b < kBoxes; ++b) {
+          int row;
           if (kGated) {
             int g = b >> 1;
             if (c.nt * p.n_step + g * 64 >= p.out_cols) g = 0;       // half-empty last tile
-            my_row = ((b & 1) ? p.sub1_base : p.sub0_base) + c.nt * p.n_step + g * 64;
+            row = ((b & 1) ? p.sub1_base : p.sub0_base) + c.nt * p.n_step + g * 64;
           } else {
-            my_row = c.nt * p.n_step + b * 64;
-            if (my_row >= p.w_rows) my_row = c.nt * p.n_step;
+            row = c.nt * p.n_step + b * 64;
+            if (row >= p.w_rows) row = c.nt * p.n_step;
           }
-          r.y = c.e * p.w_rows + my_row;
-        } else if (lane > kBoxes + 1) {
-          int rg = c.nt * Cfg::kSfbChains + (lane - kBoxes - 2);
-          if (rg >= p.sfb_rowgroups) rg = c.nt * Cfg::kSfbChains;
-          r.sf = p.sfb + (static_cast<size_t>(c.e) * p.sfb_rowgroups + rg) * p.atoms_k * 512;
+          y[b] = c.e * p.w_rows + row;
         }
-        return r;
-      };
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const LaneSrc src = locate(w);
-        const CUtensorMap* tma_a = src.tm;
-        const uint32_t a_bytes = src.a_bytes;
-        const int row0 = src.y;
-        const int my_row_y = src.y;
-        const uint8_t* my_sf = src.sf;
+        const size_t chain = static_cast<size_t>(p.atoms_k) * 512;
+        const uint8_t* sf_a = p.sfa + static_cast<size_t>(c.mt) * chain;
+        const uint8_t* sf_b[Cfg::kSfbChains];
+#pragma unroll
+        for (int g = 0; g < Cfg::kSfbChains; ++g) {
+          int rg = c.nt * Cfg::kSfbChains + g;
+          if (rg >= p.sfb_rowgroups) rg = c.nt * Cfg::kSfbChains;
+          sf_b[g] = p.sfb + (static_cast<size_t>(c.e) * p.sfb_rowgroups + rg) * chain;
+        }
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait_bounded(&tail->empty[stage], phase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
             ok = false;
             break;
           }
-          if (lane == 0) TL_STAGE(tl_k, tl_slot, TL_P_EMPTY, tl_n);
+          TL_STAGE(tl_k, tl_slot, TL_P_EMPTY, tl_n);
           const int ksteps = min(4, (p.kdim - kb * kPerStage) / kPerMma);
           // NVFP4: one scale atom per MMA step; MX: one atom covers the whole stage
           const uint32_t sf_bytes = KIND == KIND_MX ? 512u : static_cast<uint32_t>(ksteps) * 512u;
@@ -198,18 +180,17 @@ grouped_gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA,
           // the (small) scale atoms complete on a barrier of their own, so that their way into
           // TMEM starts before the operand rows of the stage have all landed
           uint64_t* sf_bar = &tail->sf_landed[stage];
-          if (lane == 0) {
-            mbar_expect_tx(bar, a_bytes + b_bytes);
-            tma_load_2d(sA + stage * kSmemA, tma_a, bar, kb * kRowBytes, row0);
-          } else if (lane <= kBoxes) {
-            tma_load_2d(sB + stage * kSmemB + (lane - 1) * 64 * kRowBytes, &tmB, bar, kb * kRowBytes, my_row_y);
-          } else if (lane == kBoxes + 1) {
-            mbar_expect_tx(sf_bar, (1u + Cfg::kSfbChains) * sf_bytes);
-            bulk_load(sSfa + stage * kSmemSfa, my_sf + sf_off, sf_bytes, sf_bar);
-          } else {
-            bulk_load(sSfb + stage * kSmemSfb + (lane - kBoxes - 2) * 2048, my_sf + sf_off, sf_bytes, sf_bar);
-          }
-          if (lane == 0) TL_STAGE(tl_k, tl_slot, TL_P_ISSUED, tl_n);
+          mbar_expect_tx(sf_bar, (1u + Cfg::kSfbChains) * sf_bytes);
+          bulk_load(sSfa + stage * kSmemSfa, sf_a + sf_off, sf_bytes, sf_bar);
+#pragma unroll
+          for (int g = 0; g < Cfg::kSfbChains; ++g)
+            bulk_load(sSfb + stage * kSmemSfb + g * 2048, sf_b[g] + sf_off, sf_bytes, sf_bar);
+          mbar_expect_tx(bar, a_bytes + b_bytes);
+#pragma unroll
+          for (int b = 0; b < kBoxes; ++b)
+            tma_load_2d(sB + stage * kSmemB + b * 64 * kRowBytes, &tmB, bar, kb * kRowBytes, y[b]);
+          tma_load_2d(sA + stage * kSmemA, tma_a, bar, kb * kRowBytes, row0);
+          TL_STAGE(tl_k, tl_slot, TL_P_ISSUED, tl_n);
           TL_INC(tl_n);
           if (++stage == kStages) {
             stage = 0;
@@ -241,7 +222,7 @@ grouped_gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA,
 #endif
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc =
           KIND == KIND_MX ? make_idesc_block_scaled(kBM, BN, /*a e4m3*/ 0, /*b e2m1*/ 5, /*ue8m0*/ 1)
                           : make_idesc_block_scaled(kBM, BN, /*a*/ 1, /*b*/ 1, /*ue4m3*/ 0);
@@ -568,6 +549,8 @@ static int gemm1_any(const b200moe_gemm_args* a, cudaStream_t stream, int tile_m
     if (p.act_kind == 0 && !(p.limit > 0.f))
       return launch_any<KIND, EPI_FC1_SILU>(bn, tmA, tmA_small, tmB, p, grid, stream);
     if (p.act_kind == 2) return launch_any<KIND, EPI_FC1_SITU>(bn, tmA, tmA_small, tmB, p, grid, stream);
+    if (p.act_kind == 1 && p.limit > 0.f)
+      return launch_any<KIND, EPI_FC1_OAI>(bn, tmA, tmA_small, tmB, p, grid, stream);
     return launch_any<KIND, EPI_FC1_GATED>(bn, tmA, tmA_small, tmB, p, grid, stream);
   }
   p.sfb_rowgroups = ceil_div_i(I, 128);

@@ -167,24 +167,21 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   regs_release_to<kRegsSmall>();
   if (warp == 0) {
     // ------------------------------ operand producer (both CTAs) -----------------
-    // lane 0: (even CTA) arms the stage barrier; token rows.  lanes 1, 2: the two 64-row boxes
-    // of this CTA's weight half.  All operand copies complete on the EVEN CTA's barrier.
-    if (lane < 3) {
-      if (lane == 0) {
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmB);
-      }
+    // One elected thread: (even CTA) arms the stage barrier; token rows, the two 64-row boxes of this
+    // CTA's weight half.  All operand copies complete on the EVEN CTA's barrier.
+    if (elect_one()) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       TL_DECL(tl_n);
       for (int w = cluster_id; ok && w < total_work; w += num_clusters) {
         const PairCoord c = decode_pair(w, p, tail, rank);
-        int y;                          // row coordinate of this lane's copy
-        if (lane == 0) {
-          y = p.mtile_row0[c.mt_load];
-        } else {
-          const int b = lane - 1;
+        const int y_a = p.mtile_row0[c.mt_load];
+        int y_b[2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
           int wrow;
           if (kGated) {
             int g = 2 * c.nt + rank;                               // pair group of this CTA
@@ -194,22 +191,20 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             wrow = c.nt * 256 + rank * 128 + b * 64;
             if (wrow >= p.w_rows) wrow = c.nt * 256 + b * 64;
           }
-          y = c.e * p.w_rows + wrow;
+          y_b[b] = c.e * p.w_rows + wrow;
         }
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait_bounded(&tail->empty[stage], phase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
             ok = false;
             break;
           }
-          if (lane == 0) TL_STAGE(tl_k, tl_slot, TL_P_EMPTY, tl_n);
+          TL_STAGE(tl_k, tl_slot, TL_P_EMPTY, tl_n);
           const uint32_t bar = map_to_cta(smem_u32(&tail->full[stage]), 0);
-          if (lane == 0) {
-            if (rank == 0) mbar_expect_tx(&tail->full[stage], stage_tx_bytes(KIND));
-            tma_load_2d_pair(sA + stage * kSmemA, &tmA, bar, kb * kRowBytes, y);
-          } else {
-            tma_load_2d_pair(sB + stage * kSmemB + (lane - 1) * 64 * kRowBytes, &tmB, bar, kb * kRowBytes, y);
-          }
-          if (lane == 0) TL_STAGE(tl_k, tl_slot, TL_P_ISSUED, tl_n);
+          if (rank == 0) mbar_expect_tx(&tail->full[stage], stage_tx_bytes(KIND));
+          tma_load_2d_pair(sA + stage * kSmemA, &tmA, bar, kb * kRowBytes, y_a);
+          tma_load_2d_pair(sB + stage * kSmemB, &tmB, bar, kb * kRowBytes, y_b[0]);
+          tma_load_2d_pair(sB + stage * kSmemB + 64 * kRowBytes, &tmB, bar, kb * kRowBytes, y_b[1]);
+          TL_STAGE(tl_k, tl_slot, TL_P_ISSUED, tl_n);
           TL_INC(tl_n);
           if (++stage == kStages) {
             stage = 0;
@@ -241,22 +236,18 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     // ------------------------------ scale-atom producer (both CTAs) --------------
     // The scale atoms travel through a ring of their own that is deeper than the operand stages:
     // they are in shared memory before the stage's tensor-memory columns are free again, so their
-    // load is off the round trip that bounds the pipeline.  lane 0: token atoms, lanes 1, 2: the
-    // two weight chains (both CTAs fetch both); they complete on this CTA's own barrier.
-    if (lane < 3) {
+    // load is off the round trip that bounds the pipeline.  Token atoms and the two weight chains
+    // (both CTAs fetch both); they complete on this CTA's own barrier.
+    if (elect_one()) {
       int slot = 0;
       uint32_t sphase = 0;
       bool ok = true;
       for (int w = cluster_id; ok && w < total_work; w += num_clusters) {
         const PairCoord c = decode_pair(w, p, tail, rank);
-        const uint8_t* my_sf;
-        if (lane == 0) {
-          my_sf = p.sfa + static_cast<size_t>(c.mt_load) * p.atoms_k * 512;
-        } else {
-          int rg = 2 * c.nt + (lane - 1);
-          if (rg >= p.sfb_rowgroups) rg = 2 * c.nt;
-          my_sf = p.sfb + (static_cast<size_t>(c.e) * p.sfb_rowgroups + rg) * p.atoms_k * 512;
-        }
+        const size_t chain = static_cast<size_t>(p.atoms_k) * 512;
+        const uint8_t* sf_a = p.sfa + static_cast<size_t>(c.mt_load) * chain;
+        const uint8_t* sf_b0 = p.sfb + (static_cast<size_t>(c.e) * p.sfb_rowgroups + 2 * c.nt) * chain;
+        const uint8_t* sf_b1 = 2 * c.nt + 1 < p.sfb_rowgroups ? sf_b0 + chain : sf_b0;
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait_bounded(&tail->sf_empty[slot], sphase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
             ok = false;
@@ -267,12 +258,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           const uint32_t sf_bytes = KIND == KIND_MX ? 512u : static_cast<uint32_t>(ksteps) * 512u;
           const size_t sf_off = static_cast<size_t>(kb) * kAtomBytes;
           uint8_t* dst = sSf + slot * kSfSlotBytes;
-          if (lane == 0) {
-            mbar_expect_tx(&tail->sf_landed[slot], 3u * sf_bytes);
-            bulk_load(dst, my_sf + sf_off, sf_bytes, &tail->sf_landed[slot]);
-          } else {
-            bulk_load(dst + kSmemSfa + (lane - 1) * 2048, my_sf + sf_off, sf_bytes, &tail->sf_landed[slot]);
-          }
+          uint64_t* bar = &tail->sf_landed[slot];
+          mbar_expect_tx(bar, 3u * sf_bytes);
+          bulk_load(dst, sf_a + sf_off, sf_bytes, bar);
+          bulk_load(dst + kSmemSfa, sf_b0 + sf_off, sf_bytes, bar);
+          bulk_load(dst + kSmemSfa + 2048, sf_b1 + sf_off, sf_bytes, bar);
           if (++slot == kSfSlots) {
             slot = 0;
             sphase ^= 1;
@@ -285,7 +275,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (even CTA) -------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc =
           KIND == KIND_MX ? make_idesc_block_scaled(256, 256, /*a e4m3*/ 0, /*b e2m1*/ 5, /*ue8m0*/ 1)
                           : make_idesc_block_scaled(256, 256, /*a*/ 1, /*b*/ 1, /*ue4m3*/ 0);
@@ -557,6 +547,7 @@ static int pair_gemm1_any(const b200moe_gemm_args* a, cudaStream_t stream) {
   if (p.act_kind == 0 && !(p.limit > 0.f))
     return pair::launch<KIND, EPI_FC1_SILU>(tmA, tmB, p, ctas, stream);
   if (p.act_kind == 2) return pair::launch<KIND, EPI_FC1_SITU>(tmA, tmB, p, ctas, stream);
+  if (p.act_kind == 1 && p.limit > 0.f) return pair::launch<KIND, EPI_FC1_OAI>(tmA, tmB, p, ctas, stream);
   return pair::launch<KIND, EPI_FC1_GATED>(tmA, tmB, p, ctas, stream);
 }
 

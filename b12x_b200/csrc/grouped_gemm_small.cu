@@ -16,7 +16,7 @@
 // loop of the next one), every epilogue warp has work when an expert holds two tokens, and the
 // tensor pipe multiplies NT columns instead of 256 mostly empty rows.
 //
-// Warp roles: warp 0 TMA producer (six lanes, one copy each per stage), warp 1 MMA issue, warps
+// Warp roles: warp 0 TMA producer, warp 1 MMA issue, warps
 // 2..9 epilogue, warp 10 copies the scale atoms of every landed stage into TMEM (tcgen05.cp) and
 // commits them to a barrier of their own.  An MMA that follows a tcgen05.cp in the SAME thread's
 // instruction stream waits out the copy's latency in the tensor pipe (about 0.15 us per dependent
@@ -146,30 +146,31 @@ grouped_gemm_nvfp4_small_kernel(const __grid_constant__ CUtensorMap tmW,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    // lane 0: arms the barrier, token rows; lanes 1, 2: the two weight sub-tiles; lane 3: token
-    // scale atoms; lanes 4, 5: weight scale atoms.
-    if (lane < 6) {
-      if (lane == 0) {
-        tma_prefetch_desc(&tmW);
-        tma_prefetch_desc(&tmX16);
-        tma_prefetch_desc(&tmX32);
-        tma_prefetch_desc(&tmX64);
-      }
+    // One elected thread issues all copies of a stage: token rows, the two weight sub-tiles, the
+    // scale atoms of the tokens and of the sub-tiles.
+    if (elect_one()) {
+      tma_prefetch_desc(&tmW);
+      tma_prefetch_desc(&tmX16);
+      tma_prefetch_desc(&tmX32);
+      tma_prefetch_desc(&tmX64);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      const int sub = (lane == 2 || lane == 5) ? 1 : 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
         const TileCoord c = decode_tile(w, p.n_tiles, tail->tile_base, p.E);
         const int row0 = p.mtile_row0[c.mt];
         const int ntok = token_cols(p.mtile_rows[c.mt]);
         const CUtensorMap* tmx = ntok == 16 ? &tmX16 : (ntok == 32 ? &tmX32 : &tmX64);
-        // first weight row (inside the expert) of this lane's sub-tile, and its scale atom chain
-        int wrow = (sub ? p.sub1_base : p.sub0_base) + c.nt * p.n_step;
-        if (wrow >= p.w_rows) wrow = p.sub0_base + c.nt * p.n_step;   // half-empty last tile
-        const uint8_t* my_sf =
-            lane == 3 ? p.sfa + static_cast<size_t>(c.mt) * p.atoms_k * 512
-                      : p.sfb + (static_cast<size_t>(c.e) * p.sfb_rowgroups + (wrow >> 7)) * p.atoms_k * 512;
+        // first weight rows (inside the expert) of the sub-tiles, and their scale atom chains
+        const int wrow0 = p.sub0_base + c.nt * p.n_step;
+        int wrow1 = p.sub1_base + c.nt * p.n_step;
+        if (wrow1 >= p.w_rows) wrow1 = wrow0;                        // half-empty last tile
+        const size_t chain = static_cast<size_t>(p.atoms_k) * 512;
+        const uint8_t* sf_x = p.sfa + static_cast<size_t>(c.mt) * chain;
+        const uint8_t* sf_e = p.sfb + static_cast<size_t>(c.e) * p.sfb_rowgroups * chain;
+        const uint8_t* sf_w0 = sf_e + static_cast<size_t>(wrow0 >> 7) * chain;
+        const uint8_t* sf_w1 = sf_e + static_cast<size_t>(wrow1 >> 7) * chain;
+        const int y0 = c.e * p.w_rows + wrow0, y1 = c.e * p.w_rows + wrow1;
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait_bounded(&tail->empty[stage], phase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
             ok = false;
@@ -179,15 +180,14 @@ grouped_gemm_nvfp4_small_kernel(const __grid_constant__ CUtensorMap tmW,
           const uint32_t sf_bytes = static_cast<uint32_t>(ksteps) * 512u;
           const size_t sf_off = static_cast<size_t>(kb) * 2048;
           uint64_t* bar = &tail->full[stage];
-          if (lane == 0) {
-            mbar_expect_tx(bar, static_cast<uint32_t>(ntok) * kRowBytes + 2u * kSmemW + 3u * sf_bytes);
-            tma_load_2d(sX + stage * kSmemX, tmx, bar, kb * kRowBytes, row0);
-          } else if (lane <= 2) {
-            tma_load_2d(sW + (stage * 2 + sub) * kSmemW, &tmW, bar, kb * kRowBytes, c.e * p.w_rows + wrow);
-          } else {
-            const int slot = lane == 3 ? 2 : sub;
-            bulk_load(sSf + (stage * 3 + slot) * kSmemSf, my_sf + sf_off, sf_bytes, bar);
-          }
+          uint8_t* sf = sSf + stage * 3 * kSmemSf;
+          mbar_expect_tx(bar, static_cast<uint32_t>(ntok) * kRowBytes + 2u * kSmemW + 3u * sf_bytes);
+          tma_load_2d(sW + stage * 2 * kSmemW, &tmW, bar, kb * kRowBytes, y0);
+          tma_load_2d(sW + (stage * 2 + 1) * kSmemW, &tmW, bar, kb * kRowBytes, y1);
+          tma_load_2d(sX + stage * kSmemX, tmx, bar, kb * kRowBytes, row0);
+          bulk_load(sf, sf_w0 + sf_off, sf_bytes, bar);
+          bulk_load(sf + kSmemSf, sf_w1 + sf_off, sf_bytes, bar);
+          bulk_load(sf + 2 * kSmemSf, sf_x + sf_off, sf_bytes, bar);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1;
@@ -201,7 +201,7 @@ grouped_gemm_nvfp4_small_kernel(const __grid_constant__ CUtensorMap tmW,
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       uint32_t acc_phase[2] = {0, 0};
@@ -259,7 +259,7 @@ grouped_gemm_nvfp4_small_kernel(const __grid_constant__ CUtensorMap tmW,
     // One thread moves the scale atoms of every landed stage from shared memory into TMEM and
     // signals their completion on a barrier of its own, so that the MMA issuer never has a
     // tensor-memory copy in front of a dependent MMA in its instruction stream.
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -332,16 +332,21 @@ grouped_gemm_nvfp4_small_kernel(const __grid_constant__ CUtensorMap tmW,
         for (int k = 0; k < 2; ++k) {
           const int ch = half + 2 * k;
           if (ch < chunks) {
+            if (p.tap != nullptr) {
+#pragma unroll
+              for (int t = 0; t < 16; ++t) {
+                if (ch * 16 + t < nrows) {
+                  float* trow = p.tap + static_cast<size_t>(row0 + ch * 16 + t) * p.w_rows + icol;
+                  trow[p.sub0_base] = __fmul_rn(__uint_as_float(ru[k][t]), alpha);
+                  trow[p.sub1_base] = __fmul_rn(__uint_as_float(rg[k][t]), alpha);
+                }
+              }
+            }
             float h[16];
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
               const float up = __fmul_rn(__uint_as_float(ru[k][t]), alpha);
               const float gate = __fmul_rn(__uint_as_float(rg[k][t]), alpha);
-              if (p.tap != nullptr && ch * 16 + t < nrows) {
-                float* trow = p.tap + static_cast<size_t>(row0 + ch * 16 + t) * p.w_rows + icol;
-                trow[p.sub0_base] = up;
-                trow[p.sub1_base] = gate;
-              }
               h[t] = round_bf16(act_gated<EPI>(gate, up, p));
             }
             uint32_t codes[2], sfw[4];
@@ -475,6 +480,7 @@ int nvfp4_small_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
   const int grid = a->num_sms > 0 ? a->num_sms : num_sms_cached();
   if (p.act_kind == 0 && !(p.limit > 0.f)) return small::launch<EPI_FC1_SILU>(tmW, tmX, p, grid, stream);
   if (p.act_kind == 2) return small::launch<EPI_FC1_SITU>(tmW, tmX, p, grid, stream);
+  if (p.act_kind == 1 && p.limit > 0.f) return small::launch<EPI_FC1_OAI>(tmW, tmX, p, grid, stream);
   return small::launch<EPI_FC1_GATED>(tmW, tmX, p, grid, stream);
 }
 
