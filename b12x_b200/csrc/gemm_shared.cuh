@@ -8,10 +8,14 @@ namespace b200moe {
 
 constexpr int kMaxExperts = 1024;
 
-// FC1 epilogues: GATED = SwiGLU with a clamp and/or the SwiGLU-OAI form (chosen at run time), SILU = plain
-// SwiGLU, SITU = the SiTU form; each is its own instantiation so that none carries the others' code.
-enum { EPI_FC1_GATED = 0, EPI_FC1_RELU2 = 1, EPI_FC2 = 2, EPI_FC1_SILU = 3, EPI_FC1_SITU = 4 };
-__host__ __device__ constexpr bool epi_is_gated(int epi) { return epi == EPI_FC1_GATED || epi == EPI_FC1_SILU || epi == EPI_FC1_SITU; }
+// FC1 epilogues: SILU = plain SwiGLU, OAI = SwiGLU-OAI with a clamp, SITU = the SiTU form, GATED = what is
+// left (SwiGLU with a clamp, SwiGLU-OAI without one, chosen at run time); each is its own instantiation
+// so that none carries the others' code: a branch per value keeps the compiler from interleaving the
+// values' chains (exponential, reciprocal), which is what an epilogue of two warps per scheduler lives on.
+enum { EPI_FC1_GATED = 0, EPI_FC1_RELU2 = 1, EPI_FC2 = 2, EPI_FC1_SILU = 3, EPI_FC1_SITU = 4, EPI_FC1_OAI = 5 };
+__host__ __device__ constexpr bool epi_is_gated(int epi) {
+  return epi == EPI_FC1_GATED || epi == EPI_FC1_SILU || epi == EPI_FC1_SITU || epi == EPI_FC1_OAI;
+}
 // KIND_NVFP4: A and B packed E2M1, E4M3 scale per 16, kind::mxf4nvf4 (K = 64 per MMA, 256 per stage).
 // KIND_MX:    A E4M3 bytes, B E2M1 expanded by TMA to one value per byte slot, E8M0 scale per 32,
 //             kind::mxf8f6f4 (K = 32 per MMA, 128 per stage; one scale atom per stage).
@@ -98,8 +102,7 @@ __device__ __forceinline__ void build_tile_base(int32_t* dst, const int32_t* __r
 // SiTU (b12x/moe/_shared/kernels/reference.py:160-172): 4 tanh(g / 4) sigmoid(g) * 25 tanh(u / 25)
 constexpr float kSituBeta = 4.0f, kSituLinearBeta = 25.0f;
 
-// EPI selects the form: EPI_FC1_SILU plain SwiGLU (no clamp); EPI_FC1_GATED clamp and/or SwiGLU-OAI, chosen
-// at run time; EPI_FC1_SITU the SiTU form.
+// EPI selects the form (see the enumeration above).
 template <int EPI>
 __device__ __forceinline__ float act_gated(float gate, float up, const GemmParams& p) {
   if (EPI == EPI_FC1_SITU) {
@@ -107,6 +110,12 @@ __device__ __forceinline__ float act_gated(float gate, float up, const GemmParam
     const float sg = __fmul_rn(__fmul_rn(kSituBeta, tanhf(__fdiv_rn(gate, kSituBeta))), s);
     const float su = __fmul_rn(kSituLinearBeta, tanhf(__fdiv_rn(up, kSituLinearBeta)));
     return __fmul_rn(sg, su);
+  }
+  if (EPI == EPI_FC1_OAI) {
+    gate = fminf(gate, p.limit);
+    up = fminf(fmaxf(up, -p.limit), p.limit);
+    const float s = rcp_newton(1.0f + expf(fminf(-(p.act_alpha * gate), 80.0f)));
+    return (gate * s) * (up + p.act_beta);
   }
   if (EPI == EPI_FC1_GATED) {
     if (p.limit > 0.f) {
@@ -125,30 +134,6 @@ __device__ __forceinline__ float act_gated(float gate, float up, const GemmParam
 
 __device__ __forceinline__ float round_bf16(float v) {
   return __bfloat162float(__float2bfloat16_rn(v));
-}
-
-// MXFP8 quantisation of 32 values (b12x/_lib/intrinsics.py:223-265): E8M0 byte = exponent of
-// pow2_ceil(amax / 448), payload = e4m3_rn_sat(x * 2^(127 - byte)).
-__device__ __forceinline__ void requant_block32_mx(const float (&v)[32], uint32_t (&o)[8],
-                                                   uint8_t& sf_byte) {
-  float amax = 0.f;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
-  uint32_t bits = __float_as_uint(__fmul_rn(amax, static_cast<float>(1.0 / 448.0)));
-  if (bits & 0x007fffffu) bits = (bits + 0x00800000u) & 0x7f800000u;
-  sf_byte = static_cast<uint8_t>((bits >> 23) & 0xffu);
-  const int ex = 254 - static_cast<int>(sf_byte);
-  const float inv = sf_byte == 0 ? 0.f : __uint_as_float(static_cast<uint32_t>(ex < 0 ? 0 : ex) << 23);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    uint32_t acc = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float q = fminf(fmaxf(__fmul_rn(v[4 * j + k], inv), -448.f), 448.f);
-      acc |= static_cast<uint32_t>(f32_to_e4m3_rn_sat(q)) << (8 * k);
-    }
-    o[j] = acc;
-  }
 }
 
 // n scale bytes (n = 1, 2 or 4, packed in `word`) -> the tile's atom chain at scale column `col`
@@ -197,6 +182,14 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int e, int mt
     // the intermediate columns col0 .. col0 + 63
     const int col0 = nt * 128 + half * 64;
     const bool cols_ok = col0 < p.out_cols;
+    if (p.tap != nullptr && valid && cols_ok) {
+      float* trow = p.tap + pos * p.w_rows + col0;
+#pragma unroll
+      for (int i = 0; i < 64; ++i) {
+        trow[p.sub0_base + i] = __fmul_rn(__uint_as_float(acc[i]), alpha);
+        trow[p.sub1_base + i] = __fmul_rn(__uint_as_float(acc[64 + i]), alpha);
+      }
+    }
     if (KIND == KIND_MX) {
       // w4a8_mx: the activation output goes straight into the MXFP8 quantiser (no bf16 staging)
       uint8_t* qrow = p.out_q + pos * p.out_cols + col0;
@@ -208,16 +201,11 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int e, int mt
         for (int i = 0; i < 32; ++i) {
           const float up = __fmul_rn(__uint_as_float(acc[blk * 32 + i]), alpha);
           const float gate = __fmul_rn(__uint_as_float(acc[64 + blk * 32 + i]), alpha);
-          if (p.tap != nullptr && valid && cols_ok) {
-            float* trow = p.tap + pos * p.w_rows + col0 + blk * 32 + i;
-            trow[p.sub0_base] = up;
-            trow[p.sub1_base] = gate;
-          }
           h[i] = act_gated<EPI>(gate, up, p);
         }
         uint32_t o[8];
         uint8_t sfb;
-        requant_block32_mx(h, o, sfb);
+        quant_block32_mx(h, o, sfb);
         if (valid && cols_ok) {
           uint4* dst = reinterpret_cast<uint4*>(qrow + blk * 32);
           dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -238,11 +226,6 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int e, int mt
         for (int i = 0; i < 16; ++i) {
           const float up = __fmul_rn(__uint_as_float(acc[ch * 16 + i]), alpha);
           const float gate = __fmul_rn(__uint_as_float(acc[64 + ch * 16 + i]), alpha);
-          if (p.tap != nullptr && valid && cols_ok) {
-            float* trow = p.tap + pos * p.w_rows + col0 + ch * 16 + i;
-            trow[p.sub0_base] = up;
-            trow[p.sub1_base] = gate;
-          }
           h[i] = round_bf16(act_gated<EPI>(gate, up, p));
         }
         uint32_t lo, hi;
@@ -257,6 +240,12 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int e, int mt
   } else if (EPI == EPI_FC1_RELU2) {
     const int col0 = nt * 256 + half * 128;
     if (col0 < p.out_cols) {
+      if (p.tap != nullptr && valid) {
+        float* trow = p.tap + pos * p.w_rows + col0;
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if (col0 + (i & ~15) < p.out_cols) trow[i] = __fmul_rn(__uint_as_float(acc[i]), alpha);
+      }
       if (KIND == KIND_MX) {
         uint8_t* qrow = p.out_q + pos * p.out_cols + col0;
         uint32_t sfw = 0u;
@@ -266,14 +255,12 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int e, int mt
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             const float v = __fmul_rn(__uint_as_float(acc[blk * 32 + i]), alpha);
-            if (p.tap != nullptr && valid && col0 + blk * 32 < p.out_cols)
-              p.tap[pos * p.w_rows + col0 + blk * 32 + i] = v;
             const float r = fmaxf(v, 0.f);
             h[i] = __fmul_rn(r, r);
           }
           uint32_t o[8];
           uint8_t sfb;
-          requant_block32_mx(h, o, sfb);
+          quant_block32_mx(h, o, sfb);
           if (valid && col0 + blk * 32 < p.out_cols) {
             uint4* dst = reinterpret_cast<uint4*>(qrow + blk * 32);
             dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -293,8 +280,6 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int e, int mt
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float v = __fmul_rn(__uint_as_float(acc[ch * 16 + i]), alpha);
-            if (p.tap != nullptr && valid && col0 + ch * 16 < p.out_cols)
-              p.tap[pos * p.w_rows + col0 + ch * 16 + i] = v;
             const float r = fmaxf(v, 0.f);
             h[i] = round_bf16(__fmul_rn(r, r));
           }

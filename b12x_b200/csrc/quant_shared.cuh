@@ -102,9 +102,11 @@ __device__ __forceinline__ void quant_block32_mx(const float (&v)[32], uint32_t 
   for (int j = 0; j < 8; ++j) {
     uint32_t acc = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float s = fminf(fmaxf(__fmul_rn(v[4 * j + k], inv), -448.f), 448.f);
-      acc |= static_cast<uint32_t>(f32_to_e4m3_rn_sat(s)) << (8 * k);
+    for (int k = 0; k < 2; ++k) {
+      // two values per conversion, which saturates at +-448; the maximum maps a NaN to -448
+      const float s0 = fmaxf(__fmul_rn(v[4 * j + 2 * k], inv), -448.f);
+      const float s1 = fmaxf(__fmul_rn(v[4 * j + 2 * k + 1], inv), -448.f);
+      acc |= static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(s0, s1), __NV_SATFINITE, __NV_E4M3)) << (16 * k);
     }
     o[j] = acc;
   }
