@@ -25,12 +25,16 @@ enum { KIND_NVFP4 = 0, KIND_MX = 1 };
 // on every FULL pair of row tiles (TILES_PAIRS) and a single-CTA kernel on the row tile that is left
 // over in experts with an odd number of them (TILES_TAIL): a pair with one empty half costs a whole
 // pair's loads and MMAs, the single tile a little more than half of that on one SM instead of two.
-enum { TILES_ALL = 0, TILES_TAIL = 1, TILES_PAIRS = 2 };
+// w4a8_mx cuts the left-over tiles once more: up to kSmallTailRows rows to the small-batch kernel (one
+// tile of as many columns), fuller ones (TILES_TAIL_LARGE) to the 128-row kernel.
+enum { TILES_ALL = 0, TILES_TAIL = 1, TILES_PAIRS = 2, TILES_TAIL_LARGE = 3 };
+constexpr int kSmallTailRows = 80;
 
 struct GemmParams {
   const uint8_t* sfa;            // activation scale atoms [mtile][atoms_k][512]
   const uint8_t* sfb;            // weight scale atoms [E][rowgroups][atoms_k][512]
   const int32_t* tile_base;      // [E+1]
+  const int32_t* expert_offsets; // [E+1]
   const int32_t* mtile_expert;
   const int32_t* mtile_row0;
   const int32_t* mtile_rows;
@@ -51,7 +55,7 @@ struct GemmParams {
   int gscale_len;
   float limit, act_alpha, act_beta;
   int act_kind;                  // gated FC1: 0 SwiGLU, 1 SwiGLU-OAI, 2 SiTU
-  int tile_mode;                 // TILES_ALL / TILES_TAIL / TILES_PAIRS
+  int tile_mode;                 // TILES_ALL / TILES_TAIL / TILES_PAIRS / TILES_TAIL_LARGE
 };
 
 struct TileCoord {
@@ -78,24 +82,47 @@ __device__ __forceinline__ TileCoord decode_tile(int w, int n_tiles, const int32
 // the same through the kernel's shared-memory work list `tb` (see build_tile_base)
 __device__ __forceinline__ TileCoord decode_work(int w, const GemmParams& p, const int32_t* tb) {
   TileCoord c = decode_tile(w, p.n_tiles, tb, p.E);
-  if (p.tile_mode == TILES_TAIL) c.mt = p.tile_base[c.e + 1] - 1;   // the expert's last row tile
+  if (p.tile_mode == TILES_TAIL || p.tile_mode == TILES_TAIL_LARGE)
+    c.mt = p.tile_base[c.e + 1] - 1;   // the expert's last row tile
   return c;
+}
+
+// Exclusive prefix sums of count(e) over the experts into dst[0..E], by one warp (every lane takes a
+// contiguous span of experts; a loop of one thread costs an L2 round trip per expert).
+template <class Count>
+__device__ __forceinline__ void prefix_experts(int32_t* dst, int E, int lane, Count count) {
+  const int per = (E + 31) >> 5;
+  const int e0 = min(E, lane * per), e1 = min(E, e0 + per);
+  int n = 0;
+  for (int e = e0; e < e1; ++e) n += count(e);
+  int incl = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  int at = incl - n;
+  for (int e = e0; e < e1; ++e) {
+    dst[e] = at;
+    at += count(e);
+  }
+  if (lane == 31) dst[E] = incl;
 }
 
 // Shared-memory work list of a single-CTA kernel (all threads call it before the set-up barrier):
 // the row-tile prefix sums as they are, or the prefix sums of "has a left-over row tile".
-__device__ __forceinline__ void build_tile_base(int32_t* dst, const int32_t* __restrict__ src, int E, int tile_mode) {
-  if (tile_mode == TILES_TAIL) {
-    if (threadIdx.x == 0) {
-      int acc = 0;
-      for (int e = 0; e < E; ++e) {
-        dst[e] = acc;
-        acc += (src[e + 1] - src[e]) & 1;
-      }
-      dst[E] = acc;
-    }
+__device__ __forceinline__ void build_tile_base(int32_t* dst, const GemmParams& p) {
+  const int32_t* __restrict__ src = p.tile_base;
+  if (p.tile_mode == TILES_TAIL || p.tile_mode == TILES_TAIL_LARGE) {
+    if (threadIdx.x < 32)
+      prefix_experts(dst, p.E, static_cast<int>(threadIdx.x), [&](int e) {
+        const int tiles = src[e + 1] - src[e];
+        if ((tiles & 1) == 0) return 0;
+        if (p.tile_mode == TILES_TAIL) return 1;
+        return p.expert_offsets[e + 1] - p.expert_offsets[e] - 128 * (tiles - 1) > kSmallTailRows ? 1 : 0;
+      });
   } else {
-    for (int i = threadIdx.x; i <= E; i += blockDim.x) dst[i] = src[i];
+    for (int i = threadIdx.x; i <= p.E; i += blockDim.x) dst[i] = src[i];
   }
 }
 

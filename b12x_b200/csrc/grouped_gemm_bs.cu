@@ -95,7 +95,11 @@ grouped_gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmA,
     tail->abort_flag = 0;
     fence_mbar_init();
   }
-  build_tile_base(tail->tile_base, p.tile_base, p.E, p.tile_mode);
+  build_tile_base(tail->tile_base, p);
+  if (p.tile_mode != TILES_ALL) {      // left-over tiles: there may be none
+    __syncthreads();
+    if (tail->tile_base[p.E] == 0) return;
+  }
   if (warp == 1) {
     tmem_alloc(&tail->tmem_base, kTmemCols);
     tmem_relinquish();
@@ -480,6 +484,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmA_small,
 void fill_common(GemmParams& p, const b200moe_gemm_args* a, char* base) {
   const b200moe_scratch_layout& L = *a->layout;
   p.tile_base = reinterpret_cast<const int32_t*>(base + L.tile_base);
+  p.expert_offsets = reinterpret_cast<const int32_t*>(base + L.expert_offsets);
   p.mtile_expert = reinterpret_cast<const int32_t*>(base + L.mtile_expert);
   p.mtile_row0 = reinterpret_cast<const int32_t*>(base + L.mtile_row0);
   p.mtile_rows = reinterpret_cast<const int32_t*>(base + L.mtile_rows);

@@ -134,17 +134,13 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     mbar_init(&tail->tmem_empty, 16);
     tail->abort_flag = 0;
     fence_mbar_init();
-    // row tiles and tile pairs per expert (prefix sums)
-    int acc = 0;
-    for (int e = 0; e < p.E; ++e) {
-      const int t0 = p.tile_base[e], t1 = p.tile_base[e + 1];
-      tail->tile_base[e] = t0;
-      tail->pair_base[e] = acc;
-      acc += (t1 - t0 + (p.tile_mode == TILES_PAIRS ? 0 : 1)) >> 1;   // full pairs only, or the odd tile too
-      if (e == p.E - 1) tail->tile_base[p.E] = t1;
-    }
-    tail->pair_base[p.E] = acc;
   }
+  // row tiles and tile pairs per expert (prefix sums); full pairs only, or the odd tile too
+  for (int i = threadIdx.x; i <= p.E; i += kThreads) tail->tile_base[i] = p.tile_base[i];
+  if (warp == 2)
+    prefix_experts(tail->pair_base, p.E, lane, [&](int e) {
+      return (p.tile_base[e + 1] - p.tile_base[e] + (p.tile_mode == TILES_PAIRS ? 0 : 1)) >> 1;
+    });
   if (warp == 1) {
     tmem_alloc_pair(&tail->tmem_base, kTmemCols);
     tmem_relinquish_pair();

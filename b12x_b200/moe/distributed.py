@@ -154,6 +154,8 @@ def gemm_launches(rows: int, experts: int, recipe: str) -> int:
     each at every size, and a kernel that scales the rows of the intermediate between them."""
     if recipe == "w4a16":
         return 3
+    if recipe == "w4a8_mx" and 256 * experts <= rows < 1024 * experts:
+        return 6     # the left-over row tiles in two launches: fuller ones, small ones
     return 4 if 256 * experts <= rows < 1024 * experts else 2
 
 

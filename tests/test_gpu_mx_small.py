@@ -1,0 +1,33 @@
+"""-m gpu: the w4a8_mx small-batch kernel at the edges of its token tiles (multiples of 16 up to 80 columns, then
+tiles of 64 = halves of the plan's 128-row tiles), and the left-over row tiles of CTA-pair plans on both sides of
+the 80 rows that decide which kernel takes them."""
+
+import pytest
+import torch
+
+from b12x_b200 import synth
+from tests.gpu_utils import run_layer
+from tests.test_gpu_parity import _check_mx_layer, _mx
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(tokens, experts, hidden, inter, act):
+    """Every token on one expert: the plan's average decides the kernel, the expert's rows the tiles."""
+    shp = _mx(tokens=tokens, experts=experts, topk=1, hidden=hidden, intermediate=inter, activation=act)
+    ids = torch.full((tokens, 1), experts - 1, dtype=torch.int32)
+    _check_mx_layer(run_layer(synth.make_inputs(shp, seed=tokens + inter), topk_ids=ids, topk_weights=torch.ones(tokens, 1)))
+
+
+@pytest.mark.parametrize("tokens", [1, 15, 17, 32, 33, 48, 63, 65, 79, 80, 81, 128, 129, 192, 200])
+@pytest.mark.parametrize("hidden,inter,act", [
+    (320, 192, "swigluoai"),      # half a k-block and half a weight tile left over
+    (128, 64, "silu"),            # one k-block, one half weight tile
+])
+def test_token_tiles(tokens, hidden, inter, act):
+    _run(tokens, 4, hidden, inter, act)
+
+
+@pytest.mark.parametrize("tokens", [257, 300, 335, 336, 337, 384, 600, 640])
+def test_left_over_row_tiles(tokens):
+    _run(tokens, 1, 256, 192, "swigluoai")
