@@ -19,7 +19,7 @@
 // warps, one per TMEM sub-partition, that take the 256-value code stages in turn), warps 12..19 are
 // the epilogue, on a double-buffered accumulator.  Every wait is bounded.
 //
-// kPair: clusters of two share a tile of 256 weight rows (each CTA converts 128 into its own TMEM)
+// Pairs: clusters of two share a tile of 256 weight rows (each CTA converts 128 into its own TMEM)
 // and up to 160 token columns, of which each CTA loads half (cta_group::2).
 //
 // Conversion.  cvt.rn.f16x2.e2m1x2 turns a byte into two FP16 code values and a half2 multiply
@@ -79,20 +79,22 @@ constexpr int kMaxList = 256;               // work items a CTA decodes ahead of
 enum { TO_F16 = 0, TO_BF16_E8M0 = 1 };
 
 // A stage is what one wait and one commit of the MMA thread cover.
-// One CTA: 2 x 64 accumulator columns + 3 converted stages of four k-blocks (128 columns each).
-// Pair: 2 x 160 + 3 of two k-blocks (64 columns).
-template <bool kPair>
+// ONE: one CTA, 2 x 64 accumulator columns + 3 converted stages of four k-blocks (128 columns each).
+// PAIR_NARROW: the same on a CTA pair.  PAIR_WIDE: 2 x 160 + 3 stages of two k-blocks (64 columns).
+enum { ONE = 0, PAIR_WIDE = 1, PAIR_NARROW = 2 };
+template <int kForm>
 struct Cfg {
-  static constexpr int kMaxTok = kPair ? 160 : 64;
+  static constexpr bool kPair = kForm != ONE;
+  static constexpr int kMaxTok = kForm == PAIR_WIDE ? 160 : 64;
   static constexpr int kColStep = kPair ? 32 : 16;   // granularity of the MMA's N (cta_group::2: 32)
-  static constexpr int kStageKb = kPair ? 2 : 4;     // k-blocks per stage
+  static constexpr int kStageKb = kForm == PAIR_WIDE ? 2 : 4;   // k-blocks per stage
   static constexpr int kStageCols = 32 * kStageKb;   // TMEM columns of a converted stage
   static constexpr int kRing = 3;
   static constexpr int kRingCol = 2 * kMaxTok;
-  static constexpr int kRawStages = kPair ? 4 : 6;
-  // token rows: two k-blocks per stage (four where no tile of the launch is wider than 32 columns and
-  // one CTA works alone), as many stages as the widest tile leaves room for
-  static constexpr int kSmemTok = kPair ? 4 * 80 * 256 : 4 * 64 * 256;
+  static constexpr int kRawStages = kForm == PAIR_WIDE ? 4 : 6;
+  // token rows: two k-blocks per stage (four where a stage of A has four and no tile of the launch puts
+  // more than 32 rows into a CTA), as many stages as the widest tile leaves room for
+  static constexpr int kSmemTok = kForm == PAIR_WIDE ? 4 * 80 * 256 : 4 * 64 * 256;
   static_assert(kRingCol + kStageCols * kRing <= kTmemCols, "tensor memory");
 };
 
@@ -112,11 +114,11 @@ struct __align__(16) SmemTail {
   int32_t offs[kMaxExperts + 1];        // first sorted row of expert e
   int4 list[kMaxList];                  // this CTA's first work items: {expert, weight tile, row0, nrows}
 };
-template <bool kPair>
+template <int kForm>
 constexpr int smem_bytes() {
-  return 1024 + Cfg<kPair>::kRawStages * kSmemRaw + Cfg<kPair>::kSmemTok + static_cast<int>(sizeof(SmemTail));
+  return 1024 + Cfg<kForm>::kRawStages * kSmemRaw + Cfg<kForm>::kSmemTok + static_cast<int>(sizeof(SmemTail));
 }
-static_assert(smem_bytes<false>() <= 227 * 1024 && smem_bytes<true>() <= 227 * 1024, "shared memory of the W4A16 kernel");
+static_assert(smem_bytes<ONE>() <= 227 * 1024 && smem_bytes<PAIR_WIDE>() <= 227 * 1024, "shared memory of the W4A16 kernel");
 
 enum { EPI_FC1_GATED = 0, EPI_FC1_RELU2 = 1, EPI_FC2 = 2 };
 
@@ -145,7 +147,7 @@ struct Params {
 struct Work {
   int e, nt, row0, nrows, cols;
 };
-template <bool kPair>
+template <int kForm>
 __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTail* tail, int rank) {
   const int32_t* tb = tail->tile_base;
   const int q = w / p.n_tiles;
@@ -159,9 +161,9 @@ __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTa
   const int me = tb[lo + 1] - tb[lo];
   const int local = w - tb[lo] * p.n_tiles;
   const int nt = local / me, mt = local - nt * me;
-  c.nt = kPair ? 2 * nt + rank : nt;
+  c.nt = Cfg<kForm>::kPair ? 2 * nt + rank : nt;
   const int first = tail->offs[lo], cnt = tail->offs[lo + 1] - first;
-  constexpr int kStep = Cfg<kPair>::kColStep;
+  constexpr int kStep = Cfg<kForm>::kColStep;
   const int step = ((cnt + me - 1) / me + kStep - 1) & ~(kStep - 1);
   c.row0 = first + mt * step;
   c.nrows = min(step, cnt - mt * step);
@@ -169,11 +171,11 @@ __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTa
   return c;
 }
 // the i-th item of this CTA, w = its number: out of the list the CTA made at its start where that reaches
-template <bool kPair>
+template <int kForm>
 __device__ __forceinline__ Work get_work(int i, int w, const Params& p, const SmemTail* tail, int rank) {
-  if (i >= kMaxList) return decode_work<kPair>(w, p, tail, rank);
+  if (i >= kMaxList) return decode_work<kForm>(w, p, tail, rank);
   const int4 v = tail->list[i];
-  constexpr int kStep = Cfg<kPair>::kColStep;
+  constexpr int kStep = Cfg<kForm>::kColStep;
   Work c;
   c.e = v.x;
   c.nt = v.y;
@@ -270,12 +272,13 @@ __device__ __forceinline__ void mma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tme
       : "memory");
 }
 
-template <int EPI, bool kPair, int kTo>
+template <int EPI, int kForm, int kTo>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __grid_constant__ CUtensorMap tmX32,
                           const __grid_constant__ CUtensorMap tmX16, const __grid_constant__ CUtensorMap tmW,
                           const Params p) {
-  using C = Cfg<kPair>;
+  using C = Cfg<kForm>;
+  constexpr bool kPair = C::kPair;
   constexpr bool kGated = EPI == EPI_FC1_GATED;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -348,7 +351,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
   const int w_first = kPair ? static_cast<int>(blockIdx.x) >> 1 : static_cast<int>(blockIdx.x);
   const int w_stride = kPair ? static_cast<int>(gridDim.x) >> 1 : static_cast<int>(gridDim.x);
   if (static_cast<int>(threadIdx.x) < kMaxList && w_first + static_cast<int>(threadIdx.x) * w_stride < total_work) {
-    const Work c = decode_work<kPair>(w_first + static_cast<int>(threadIdx.x) * w_stride, p, tail, rank);
+    const Work c = decode_work<kForm>(w_first + static_cast<int>(threadIdx.x) * w_stride, p, tail, rank);
     tail->list[threadIdx.x] = make_int4(c.e, c.nt, c.row0, c.nrows);
   }
   __syncthreads();
@@ -359,7 +362,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
   volatile int* abort_flag = &tail->abort_flag;
   // a k-block of the widest tile's token rows (of this CTA's share), k-blocks per stage, stages
   const int tok_kb_bytes = (kPair ? tail->max_cols >> 1 : tail->max_cols) * 128;
-  const int tok_kbs = (!kPair && tail->max_cols <= 32) ? 4 : 2;
+  const int tok_kbs = C::kStageKb == 4 && tok_kb_bytes <= 32 * 128 ? 4 : 2;
   const int tok_stages = min(kTokStagesMax, C::kSmemTok / (tok_kbs * tok_kb_bytes));
 
   if (warp == 0) {
@@ -373,7 +376,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       uint32_t rphase = 0;
       bool ok = true;
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kPair>(it, w, p, tail, rank);
+        const Work c = get_work<kForm>(it, w, p, tail, rank);
         const int nt = min(c.nt, p.n_row_tiles - 1);        // half-empty last pair: load the other half again
         const int r0 = p.sub0_base + nt * p.n_step;
         int r1 = p.sub1_base + nt * p.n_step;
@@ -422,7 +425,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       uint32_t tphase = 0;
       bool ok = true;
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kPair>(it, w, p, tail, rank);
+        const Work c = get_work<kForm>(it, w, p, tail, rank);
         const int rows = kPair ? c.cols >> 1 : c.cols;       // 16, 32, 48, 64 or 80
         const int big = rows >= 64 ? 64 : (rows & 32);
         const CUtensorMap* tm = big == 64 ? &tmX64 : &tmX32;
@@ -466,7 +469,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       bool ok = true;
       const uint64_t bdesc0 = make_desc_sw128(smem_u32(sTok));
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kPair>(it, w, p, tail, rank);
+        const Work c = get_work<kForm>(it, w, p, tail, rank);
         const uint32_t idesc = make_idesc_16bit(kPair ? 256 : 128, c.cols, kTo != TO_F16);
         if (!mbar_wait_bounded(&tail->acc_empty[buf], acc_phase[buf] ^ 1, abort_flag, p.status, WAIT_TMEM_EMPTY)) {
           ok = false;
@@ -518,7 +521,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
             }
           }
         };
-        if (!kPair && tok_kbs == 4) main_loop(std::integral_constant<int, kPair ? 2 : 4>{});
+        if (tok_kbs == 4) main_loop(std::integral_constant<int, C::kStageKb>{});
         else main_loop(std::integral_constant<int, 2>{});
         if (ok) {
           if (kPair) tc_commit_pair_both(&tail->acc_full[buf]);
@@ -542,7 +545,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
     uint32_t raw0 = 0, stage0 = 0;   // raw stages and MMA stages before this tile
     bool ok = true;
     for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-      const Work c = get_work<kPair>(it, w, p, tail, rank);
+      const Work c = get_work<kForm>(it, w, p, tail, rank);
       const int nt = min(c.nt, p.n_row_tiles - 1);
       const int r0 = p.sub0_base + nt * p.n_step;
       int r1 = p.sub1_base + nt * p.n_step;
@@ -641,7 +644,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
     uint32_t acc_phase[2] = {0, 0};
     int buf = 0;
     for (int w = w_first, it = 0; w < total_work; w += w_stride, ++it) {
-      const Work c = get_work<kPair>(it, w, p, tail, rank);
+      const Work c = get_work<kForm>(it, w, p, tail, rank);
       const float alpha = p.alphas[c.e];
       // lane l holds the factors of token t + l of the warp's next 32 (FC2: 16) columns; the first are
       // fetched before the accumulator is waited for
@@ -928,10 +931,11 @@ static int make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t cols, uin
   return r == CUDA_SUCCESS ? B200MOE_OK : B200MOE_ECUDA;
 }
 
-template <int EPI, bool kPair, int kTo>
+template <int EPI, int kForm, int kTo>
 static int launch(const CUtensorMap (&tmX)[3], const CUtensorMap& tmW, const Params& p, int ctas, cudaStream_t s) {
-  auto kern = grouped_gemm_w4a16_kernel<EPI, kPair, kTo>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<kPair>()) != cudaSuccess)
+  constexpr bool kPair = Cfg<kForm>::kPair;
+  auto kern = grouped_gemm_w4a16_kernel<EPI, kForm, kTo>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<kForm>()) != cudaSuccess)
     return B200MOE_ECUDA;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr;
@@ -941,7 +945,7 @@ static int launch(const CUtensorMap (&tmX)[3], const CUtensorMap& tmW, const Par
   attr.val.clusterDim.z = 1;
   cfg.gridDim = dim3(static_cast<unsigned>(kPair ? ctas & ~1 : ctas));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem_bytes<kPair>();
+  cfg.dynamicSmemBytes = smem_bytes<kForm>();
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
@@ -954,19 +958,21 @@ static int launch(const CUtensorMap (&tmX)[3], const CUtensorMap& tmW, const Par
   return cudaLaunchKernelEx(&cfg, kern, tmX[0], tmX[1], tmX[2], tmW, p) == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }
 
-// Pairs from a plan average of 32 rows per expert on: the pair's token tiles are wider (160 columns
-// against 64) and it loads each token row half as often, one CTA has finer tiles and no partner to wait
-// for.  FC1 + FC2 of the Qwen3 shape at 24 / 32 / 48 rows per expert, one CTA against pairs: 359 : 368,
-// 378 : 375, 398 : 390 us; at 4 and 16 rows 269 : 365 and 281 : 368; at 256 rows 1657 : 1017.
-// B200MOE_W4A16_PAIR=1 / 0 forces pairs on / off.
-static bool use_pair(const b200moe_gemm_args* a) {
+// One CTA up to 18 rows per expert (finer tiles, no partner to wait for), narrow pairs to 58 (nearly every
+// expert is one tile of at most 64 columns; one wait of the MMA thread covers 256 rows x 256 values), wide
+// pairs beyond.  FC1 + FC2 of the Qwen3 shape, one CTA : narrow : wide, in us: 1 row per expert 185 : 200 :
+// 249, 16 rows 283 : 290 : 366, 24 rows 360 : 296 : 368, 48 rows 397 : 323 : 387, 56 rows 447 : 361 : 401,
+// 64 rows 564 : 444 : 421, 88 rows 759 : 583 : 454.
+// B200MOE_W4A16_PAIR=1 / 0 forces wide pairs / one CTA (2: narrow pairs).
+static int form_for(const b200moe_gemm_args* a) {
   static int mode = -2;
   if (mode == -2) {
     const char* e = getenv("B200MOE_W4A16_PAIR");
-    mode = e == nullptr ? -1 : (atoi(e) != 0 ? 1 : 0);
+    mode = e == nullptr ? -1 : atoi(e);
   }
-  if (mode >= 0) return mode == 1;
-  return static_cast<int64_t>(a->layout->rows) >= 32ll * a->num_experts;
+  if (mode >= 0) return mode == 0 ? ONE : (mode == 2 ? PAIR_NARROW : PAIR_WIDE);
+  const int64_t rows = a->layout->rows, experts = a->num_experts;
+  return rows < 18 * experts ? ONE : (rows < 58 * experts ? PAIR_NARROW : PAIR_WIDE);
 }
 
 template <int EPI, int kTo>
@@ -981,12 +987,11 @@ static int launch_any(const b200moe_gemm_args* a, const void* tokens, uint64_t c
   const int rc = make_tmap_bytes_2d(&tmW, weights, cols / 2, static_cast<uint64_t>(a->num_experts) * p.w_rows, 64);
   if (rc != B200MOE_OK) return rc;
   const int ctas = a->num_sms > 0 ? a->num_sms : num_sms_cached();
-  if (use_pair(a)) {
-    p.n_tiles = ceil_div_i(p.n_row_tiles, 2);
-    return launch<EPI, true, kTo>(tmX, tmW, p, ctas, s);
-  }
-  p.n_tiles = p.n_row_tiles;
-  return launch<EPI, false, kTo>(tmX, tmW, p, ctas, s);
+  const int form = form_for(a);
+  p.n_tiles = form == ONE ? p.n_row_tiles : ceil_div_i(p.n_row_tiles, 2);
+  if (form == ONE) return launch<EPI, ONE, kTo>(tmX, tmW, p, ctas, s);
+  if (form == PAIR_NARROW) return launch<EPI, PAIR_NARROW, kTo>(tmX, tmW, p, ctas, s);
+  return launch<EPI, PAIR_WIDE, kTo>(tmX, tmW, p, ctas, s);
 }
 
 // one warp per row, eight per CTA

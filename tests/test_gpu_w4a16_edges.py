@@ -1,5 +1,5 @@
 """-m gpu: the W4A16 kernels at the edges of their token tiles (16-column steps on one CTA, at most 64; 32-column
-steps on a CTA pair, at most 160), of their stages (two and four k-blocks of 64) and of their weight tiles, and the
+steps on a CTA pair, at most 64 or 160), of their stages (two and four k-blocks of 64) and of their weight tiles, and the
 per-row power-of-two scaling of the FP16 token rows over the range of BF16."""
 
 from dataclasses import replace
@@ -28,7 +28,15 @@ def test_single_cta_token_tiles(tokens, hidden, inter):
     _check_w4a16_layer(run_layer(inp, topk_ids=ids, topk_weights=w))
 
 
-@pytest.mark.parametrize("tokens", [32, 33, 160, 161, 320, 321, 500])
+@pytest.mark.parametrize("tokens", [18, 32, 33, 57, 80, 115, 128, 150])
+@pytest.mark.parametrize("hidden,inter", [(64, 64), (320, 192), (256, 128)])
+def test_narrow_pair_token_tiles(tokens, hidden, inter):
+    """Plans of 18 to 57 rows per expert (four experts above that many rows, all on one of them)."""
+    inp, ids, w = _one_expert(tokens, 1 if tokens < 58 else 4, hidden, inter)
+    _check_w4a16_layer(run_layer(inp, topk_ids=ids, topk_weights=w))
+
+
+@pytest.mark.parametrize("tokens", [58, 160, 161, 320, 321, 500])
 @pytest.mark.parametrize("hidden,inter,act", [(64, 64, "silu"), (448, 320, "silu"), (192, 192, "relu2")])
 def test_cta_pair_token_tiles(tokens, hidden, inter, act):
     inp, ids, w = _one_expert(tokens, 1, hidden, inter, act)
