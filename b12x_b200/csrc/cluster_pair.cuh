@@ -57,21 +57,6 @@ __device__ __forceinline__ void tc_commit_pair_both(uint64_t* bar) {
       ::"r"(smem_u32(bar)), "h"(mask)
       : "memory");
 }
-// Arrive on a barrier of another CTA of the cluster after shared-memory writes of this thread (made
-// visible to the tensor core's proxy by fence.proxy.async before the call): release semantics.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// D[tmem of both CTAs] (+)= A[smem, 128 rows per CTA] * B[smem, half of N per CTA], kind::f16
-__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 
 }  // namespace pair
 }  // namespace b200moe
