@@ -84,9 +84,7 @@ extern "C" int b200moe_scratch_nbytes(const b200moe_caps* c, b200moe_scratch_lay
       break;
     case B200MOE_RECIPE_W4A16:
       if (K % 32 != 0 || I % 32 != 0) return B200MOE_EINVAL;
-      // 16-bit rows in sorted order (x for FC1, then the FP16 form of the intermediate for FC2), bf16
-      // intermediate
-      act_row = (K > I ? K : I) * 2; mid_row = I * 2;
+      act_row = K * 2; mid_row = I * 2;   // bf16 rows in sorted order, bf16 intermediate
       break;
     default:
       return B200MOE_EINVAL;
@@ -107,10 +105,12 @@ extern "C" int b200moe_scratch_nbytes(const b200moe_caps* c, b200moe_scratch_lay
   L->sorted_route_ids = take(rows64 * 4);
   L->inv_perm = take(rows64 * 4);
   L->act_q = take(rows64 * act_row);
-  // w4a16 has no activation scales: its region holds the power-of-two factors of the sorted rows, FC1's and FC2's
-  L->act_sf = take(c->recipe == B200MOE_RECIPE_W4A16 ? rows64 * 8 : mtile_cap * act_atoms * 512);
+  // w4a16 has no activation scales.  Its two scale regions hold what the GEMMs make of the sorted rows: act_sf
+  // the rows' power-of-two factors (FC1's, then FC2's), mid_sf the rows as FP16 (FC1's, later FC2's).
+  const bool w4a16 = c->recipe == B200MOE_RECIPE_W4A16;
+  L->act_sf = take(w4a16 ? rows64 * 8 : mtile_cap * act_atoms * 512);
   L->mid_q = take(rows64 * mid_row);
-  L->mid_sf = take(mtile_cap * mid_atoms * 512);
+  L->mid_sf = take(w4a16 ? rows64 * (K > I ? K : I) * 2 : mtile_cap * mid_atoms * 512);
   L->routed = take(rows64 * K * 4);
   L->sort_tmp = take(((rows64 + 2047) / 2048) * E * 4);
   L->total_nbytes = off;

@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(256) activation_amax_kernel(
     const __nv_bfloat16* __restrict__ rows_fc1, const __nv_bfloat16* __restrict__ rows_fc2, int K, int I,
     const int32_t* __restrict__ tile_base, int E, const int32_t* __restrict__ mtile_expert,
     const int32_t* __restrict__ mtile_row0, const int32_t* __restrict__ mtile_rows, float* __restrict__ amax,
-    int layer_idx, const float* __restrict__ row_inv) {
+    int layer_idx) {
   const int mt = blockIdx.x;
   if (mt >= tile_base[E]) return;
   const int which = blockIdx.y;
@@ -796,18 +796,11 @@ __global__ void __launch_bounds__(256) activation_amax_kernel(
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
     const uint4 p = reinterpret_cast<const uint4*>(base)[i];
     const uint32_t w[4] = {p.x, p.y, p.z, p.w};
-    // FC1 rows are held as FP16, scaled per row, or (factor 0) as BF16
-    const float inv = which == 0 ? row_inv[mtile_row0[mt] + i / (len >> 3)] : 0.f;
-    const bool f16 = inv != 0.f;
-    float v = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float2 f = f16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j]))
-                           : make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
-      v = fmaxf(v, fmaxf(fabsf(f.x), fabsf(f.y)));
+      m = fmaxf(m, fabsf(__uint_as_float(w[j] << 16)));
+      m = fmaxf(m, fabsf(__uint_as_float(w[j] & 0xffff0000u)));
     }
-    if (f16) v = __fmul_rn(v, inv);
-    m = fmaxf(m, v);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -824,40 +817,41 @@ __global__ void __launch_bounds__(256) activation_amax_kernel(
   }
 }
 
-// x rows -> sorted-position order (the token operand of FC1), one warp per row; row_inv[pos] = 0 marks
-// them as BF16 values as they were.
+// x rows -> sorted-position order (the token operand of FC1), one warp per row
 __global__ void __launch_bounds__(256) permute_rows_bf16_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* __restrict__ expert_offsets,
     int E, const int32_t* __restrict__ sorted_route_ids, int num_topk, int K,
-    __nv_bfloat16* __restrict__ out, float* __restrict__ row_inv) {
+    __nv_bfloat16* __restrict__ out) {
   const int total = expert_offsets[E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int pos = blockIdx.x * 8 + warp; pos < total; pos += gridDim.x * 8) {
     const int tkn = sorted_route_ids[pos] / num_topk;
-    if (lane == 0) row_inv[pos] = 0.f;
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(tkn) * x_row_stride);
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(pos) * K);
     for (int j = lane; j < (K >> 3); j += 32) dst[j] = __ldg(src + j);
   }
 }
 
-// The same rows (sorted_route_ids null: rows that lie in sorted order already, FC2's) as FP16, each multiplied by the power of two that puts its largest finite magnitude
+// The same, and the rows once more as FP16 (rows_bf16 and sorted_route_ids null: rows that lie in sorted order
+// already, FC2's, as FP16 only), each multiplied by the power of two that puts its largest finite magnitude
 // into [2^14, 2^15); row_inv[pos] takes the inverse.  BF16 has 8 significant bits: every value down
 // to 2^-32 of the row's largest is carried over exactly, anything smaller to within 2^-40 of it,
 // far below one rounding of the FP32 accumulator.  Infinities and NaNs stay what they are.
 __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* __restrict__ expert_offsets,
-    int E, const int32_t* __restrict__ sorted_route_ids, int num_topk, int K, __half* __restrict__ out,
-    float* __restrict__ row_inv) {
+    int E, const int32_t* __restrict__ sorted_route_ids, int num_topk, int K,
+    __nv_bfloat16* __restrict__ rows_bf16, __half* __restrict__ out, float* __restrict__ row_inv) {
   const int total = expert_offsets[E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = K >> 3;
   for (int pos = blockIdx.x * 8 + warp; pos < total; pos += gridDim.x * 8) {
     const int tkn = sorted_route_ids != nullptr ? sorted_route_ids[pos] / num_topk : pos;
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(tkn) * x_row_stride);
+    uint4* copy = rows_bf16 != nullptr ? reinterpret_cast<uint4*>(rows_bf16 + static_cast<size_t>(pos) * K) : nullptr;
     __nv_bfloat162 m2 = __float2bfloat162_rn(0.f);
     for (int j = lane; j < nvec; j += 32) {
       const uint4 v = __ldg(src + j);
+      if (copy != nullptr) copy[j] = v;
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
@@ -1032,11 +1026,13 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
   if (f16)
     permute_rows_f16_kernel<<<ggrid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes, a->num_topk, K,
-        reinterpret_cast<__half*>(base + L.act_q), reinterpret_cast<float*>(base + L.act_sf));
+        reinterpret_cast<__nv_bfloat16*>(base + L.act_q), reinterpret_cast<__half*>(base + L.mid_sf),
+        reinterpret_cast<float*>(base + L.act_sf));
   else
     permute_rows_bf16_kernel<<<ggrid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes, a->num_topk, K,
-        reinterpret_cast<__nv_bfloat16*>(base + L.act_q), reinterpret_cast<float*>(base + L.act_sf));
+        reinterpret_cast<__nv_bfloat16*>(base + L.act_q));
+  const void* tokens = base + (f16 ? L.mid_sf : L.act_q);
   Params p = {};
   fill_common(p, a, base);
   p.sf = a->w13_sf;
@@ -1057,15 +1053,15 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
     p.n_step = 64;
     p.sub0_base = a->gate_first ? I : 0;   // up rows
     p.sub1_base = a->gate_first ? 0 : I;   // gate rows
-    return f16 ? launch_any<EPI_FC1_GATED, TO_F16>(a, base + L.act_q, K, a->w13, p, stream)
-               : launch_any<EPI_FC1_GATED, TO_BF16_E8M0>(a, base + L.act_q, K, a->w13, p, stream);
+    return f16 ? launch_any<EPI_FC1_GATED, TO_F16>(a, tokens, K, a->w13, p, stream)
+               : launch_any<EPI_FC1_GATED, TO_BF16_E8M0>(a, tokens, K, a->w13, p, stream);
   }
   p.n_row_tiles = ceil_div_i(I, 128);
   p.n_step = 128;
   p.sub0_base = 0;
   p.sub1_base = 64;
-  return f16 ? launch_any<EPI_FC1_RELU2, TO_F16>(a, base + L.act_q, K, a->w13, p, stream)
-             : launch_any<EPI_FC1_RELU2, TO_BF16_E8M0>(a, base + L.act_q, K, a->w13, p, stream);
+  return f16 ? launch_any<EPI_FC1_RELU2, TO_F16>(a, tokens, K, a->w13, p, stream)
+             : launch_any<EPI_FC1_RELU2, TO_BF16_E8M0>(a, tokens, K, a->w13, p, stream);
 }
 
 int w4a16_gemm2(const b200moe_gemm_args* a, cudaStream_t stream) {
@@ -1090,14 +1086,14 @@ int w4a16_gemm2(const b200moe_gemm_args* a, cudaStream_t stream) {
   p.sub0_base = 0;
   p.sub1_base = 64;
   if (a->sf_e8m0) return launch_any<EPI_FC2, TO_BF16_E8M0>(a, base + L.mid_q, I, a->w2, p, stream);
-  // the intermediate rows as FP16, in the place of FC1's token rows
+  // the intermediate rows as FP16, in the place of FC1's
   const int rows = a->num_tokens * a->num_topk;
   float* row_inv = reinterpret_cast<float*>(base + L.act_sf) + L.rows;
   permute_rows_f16_kernel<<<row_grid(rows), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(base + L.mid_q), I, p.expert_offsets, E, nullptr, 1, I,
-      reinterpret_cast<__half*>(base + L.act_q), row_inv);
+      reinterpret_cast<const __nv_bfloat16*>(base + L.mid_q), I, p.expert_offsets, E, nullptr, 1, I, nullptr,
+      reinterpret_cast<__half*>(base + L.mid_sf), row_inv);
   p.row_inv = row_inv;
-  return launch_any<EPI_FC2, TO_F16>(a, base + L.act_q, I, a->w2, p, stream);
+  return launch_any<EPI_FC2, TO_F16>(a, base + L.mid_sf, I, a->w2, p, stream);
 }
 
 int w4a16_activation_amax(const b200moe_amax_args* a, cudaStream_t stream) {
@@ -1111,8 +1107,7 @@ int w4a16_activation_amax(const b200moe_amax_args* a, cudaStream_t stream) {
       reinterpret_cast<const __nv_bfloat16*>(base + L.act_q), reinterpret_cast<const __nv_bfloat16*>(base + L.mid_q),
       a->hidden_size, a->intermediate, reinterpret_cast<const int32_t*>(base + L.tile_base), a->num_experts,
       reinterpret_cast<const int32_t*>(base + L.mtile_expert), reinterpret_cast<const int32_t*>(base + L.mtile_row0),
-      reinterpret_cast<const int32_t*>(base + L.mtile_rows), a->amax, a->layer_idx,
-      reinterpret_cast<const float*>(base + L.act_sf));
+      reinterpret_cast<const int32_t*>(base + L.mtile_rows), a->amax, a->layer_idx);
   return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }
 

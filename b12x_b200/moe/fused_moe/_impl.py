@@ -783,8 +783,9 @@ class TPMoEFP4Binding:
 
     @property
     def packed_input_scale(self) -> torch.Tensor:
-        per = {"nvfp4": 64, "w4a8_mx": 128, "w4a16": 64}[self.quant_mode]
-        atoms = (self.k + per - 1) // per
+        if self.quant_mode == "w4a16":          # bf16 rows have no scales
+            return self._v("act_sf", 0, torch.uint8)
+        atoms = -(-self.k // (64 if self.quant_mode == "nvfp4" else 128))
         return self._v("act_sf", self.core_layout.mtile_cap * atoms * 512, torch.uint8)
 
     @property
@@ -794,8 +795,9 @@ class TPMoEFP4Binding:
 
     @property
     def intermediate_scale(self) -> torch.Tensor:
-        per = {"nvfp4": 64, "w4a8_mx": 128, "w4a16": 64}[self.quant_mode]
-        atoms = (self.n + per - 1) // per
+        if self.quant_mode == "w4a16":
+            return self._v("mid_sf", 0, torch.uint8)
+        atoms = -(-self.n // (64 if self.quant_mode == "nvfp4" else 128))
         return self._v("mid_sf", self.core_layout.mtile_cap * atoms * 512, torch.uint8)
 
     @property

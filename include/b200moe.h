@@ -78,9 +78,10 @@ typedef struct {
   int64_t sorted_route_ids;  /* int32[rows]  flat route id (t*k+slot) per position */
   int64_t inv_perm;          /* int32[rows]  position per flat route id, -1 = dropped */
   int64_t act_q;             /* FC1 input: codes [rows][K/2] (nvfp4) / [rows][K] (mxfp8) / bf16 [rows][K] (w4a16) */
-  int64_t act_sf;            /* FC1 input scales, 512-byte atoms [mtile_cap][ceil(K/64|128)]  */
+  int64_t act_sf;            /* FC1 input scales, 512-byte atoms [mtile_cap][ceil(K/64|128)]; w4a16 (no scales): float32
+                                [2][rows], the power-of-two factors of FC1's and FC2's FP16 rows */
   int64_t mid_q;             /* FC2 input codes  [rows][I/2] / [rows][I] / bf16 [rows][I]     */
-  int64_t mid_sf;            /* FC2 input scales atoms                                         */
+  int64_t mid_sf;            /* FC2 input scales atoms; w4a16: work space, FP16 rows [rows][max(K,I)] */
   int64_t routed;            /* float32 [rows][K] per-route FC2 output (alpha applied)         */
   int64_t sort_tmp;          /* int32 [ceil(rows/2048)][E] per-chunk counts of the multi-CTA sort */
   int32_t rows;              /* T*k                                             */
@@ -272,7 +273,8 @@ int b200moe_grouped_gemm1_act(const b200moe_gemm_args* a, void* stream);
 int b200moe_grouped_gemm2(const b200moe_gemm_args* a, void* stream);
 
 /* Calibration side channel (w4a16 only, as in the reference: b12x/moe/fused_moe/_impl.py:10601-10604,
- * w4a16/kernel.py:7288-7365).  After b200moe_grouped_gemm1_act of the same arguments:
+ * w4a16/kernel.py:7288-7365).  After b200moe_grouped_gemm1_act of the same arguments, before or after
+ * b200moe_grouped_gemm2:
  * amax[layer_idx][e][0] = max(old, max |x| over the rows routed to local expert e),
  * amax[layer_idx][e][1] = the same over the expert's activated BF16 intermediate rows.
  * amax is a device float32 [layers][num_experts][2] that the caller zeroes once. */

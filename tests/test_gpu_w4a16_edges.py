@@ -2,12 +2,14 @@
 steps on a CTA pair, at most 64 or 160), of their stages (two and four k-blocks of 64) and of their weight tiles, and the
 per-row power-of-two scaling of the FP16 token rows over the range of BF16."""
 
+import ctypes as C
 from dataclasses import replace
 
 import pytest
 import torch
 
 from b12x_b200 import synth
+from b12x_b200._lib import ext
 from tests.gpu_utils import oracle_layer, run_layer
 from tests.test_gpu_parity import _check_w4a16_layer, _w16
 
@@ -76,3 +78,25 @@ def test_row_scaling_over_the_bf16_range():
     keep = [i for i in range(48) if i not in (5, 40)]
     assert torch.equal(again.out_f32[keep], run.out_f32[keep])
     assert not bool(torch.isfinite(again.out_f32[5]).any()) and bool(torch.isnan(again.out_f32[40]).all())
+
+
+@pytest.mark.parametrize("tokens,hidden,inter", [(40, 256, 128), (150, 192, 448)])      # wider and narrower than I
+def test_token_rows_are_readable_after_a_run(tokens, hidden, inter):
+    """``packed_input`` holds the sorted BF16 rows after the whole layer, and the calibration maxima taken after FC2
+    equal those of the BF16 rows; there are no activation scales to read."""
+    shp = _w16(tokens=tokens, experts=5, topk=2, hidden=hidden, intermediate=inter)
+    run = run_layer(synth.make_inputs(shp, seed=tokens))
+    b, rows = run.binding, tokens * 2
+    x = run.inp.x.cpu()[(b.packed_route_indices.cpu() // 2).long()]
+    assert torch.equal(b.packed_input.cpu()[:rows].view(torch.bfloat16), x)
+    assert b.packed_input_scale.numel() == 0 and b.intermediate_scale.numel() == 0
+    amax = torch.zeros(1, 5, 2, device="cuda")
+    args = ext.AmaxArgs(b.kernel_workspace.data_ptr(), C.pointer(b.core_layout), amax.data_ptr(), rows, 5, hidden, inter, 0,
+                        ext.RECIPES["w4a16"])
+    ext.check(ext.load().b200moe_activation_amax(C.byref(args), torch.cuda.current_stream().cuda_stream), "amax")
+    mid = b.materialized_intermediate.cpu()[:rows].view(torch.bfloat16).float()
+    offs = b.expert_offsets.cpu().tolist()
+    for e in range(5):
+        for which, v in enumerate((x.float(), mid)):
+            part = v[offs[e]:offs[e + 1]].abs()
+            assert amax[0, e, which].item() == (part.max().item() if part.numel() else 0.0)
