@@ -96,7 +96,7 @@ extern "C" int b200moe_scratch_nbytes(const b200moe_caps* c, b200moe_scratch_lay
     return o;
   };
   L->status = take(16 * 4);
-  L->expert_counts = take(E * 4);
+  L->expert_counts = take(3 * E * 4);   // counts, then the marks the sort clears for w4a16
   L->expert_offsets = take((E + 1) * 4);
   L->tile_base = take((E + 1) * 4);
   L->mtile_expert = take(mtile_cap * 4);

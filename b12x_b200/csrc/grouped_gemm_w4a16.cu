@@ -27,7 +27,9 @@
 // takes three more (FP16 -> FP32 twice, pack), and that sequence tops out at 36 to 39 values per
 // clock and SM against 70 to 77; so the MMA runs on FP16 x FP16 and the token rows come as FP16,
 // scaled by a power of two per row (permute_rows_f16_kernel), which BF16 values survive unchanged.
-// E8M0 scales exceed the FP16 range: with them both operands are BF16.
+// E8M0 scales exceed the FP16 range: with them both operands are BF16.  So they are for an expert one of
+// whose rows spans more binades than FP16 carries exactly (permute_rows_f16_kernel marks it): its items
+// take the BF16 rows and re-encode the weights, at the lower rate.
 //
 // What bounds it and what it took, on the Qwen3-235B shape (K 4096, I 1536, 128 experts, top-8),
 // FC1 / FC2 in microseconds:
@@ -112,7 +114,7 @@ struct __align__(16) SmemTail {
   int max_cols;                         // of all tiles of the launch
   int32_t tile_base[kMaxExperts + 1];   // token tiles before expert e
   int32_t offs[kMaxExperts + 1];        // first sorted row of expert e
-  int4 list[kMaxList];                  // this CTA's first work items: {expert, weight tile, row0, nrows}
+  int4 list[kMaxList];                  // this CTA's first work items: {expert (+ kWideBit), weight tile, row0, nrows}
 };
 template <int kForm>
 constexpr int smem_bytes() {
@@ -140,14 +142,23 @@ struct Params {
   float limit, act_alpha, act_beta;
   int swigluoai;
   const float* row_inv;          // TO_F16: per sorted row, the power of two that undoes its scaling
+  const int32_t* wide;           // TO_F16: per expert, nonzero = BF16 operands
+};
+
+// Token rows, one map per box height: 64, 32 and 16 rows.  [0] the rows as `kTo` says, [1] TO_F16: the
+// same rows as BF16, for experts marked `wide`.
+struct TokenMaps {
+  CUtensorMap m[2][3];
 };
 
 // A work item: expert, weight tile, and the token rows [row0, row0 + nrows) of the expert.  An
 // expert's rows are cut evenly into as few tiles as the column limit allows.
 struct Work {
   int e, nt, row0, nrows, cols;
+  bool wide;
 };
-template <int kForm>
+constexpr int kWideBit = 1 << 16;      // of a listed item's expert
+template <int kForm, int kTo>
 __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTail* tail, int rank) {
   const int32_t* tb = tail->tile_base;
   const int q = w / p.n_tiles;
@@ -168,16 +179,18 @@ __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTa
   c.row0 = first + mt * step;
   c.nrows = min(step, cnt - mt * step);
   c.cols = (c.nrows + kStep - 1) & ~(kStep - 1);
+  c.wide = kTo == TO_F16 && p.wide[lo] != 0;
   return c;
 }
 // the i-th item of this CTA, w = its number: out of the list the CTA made at its start where that reaches
-template <int kForm>
+template <int kForm, int kTo>
 __device__ __forceinline__ Work get_work(int i, int w, const Params& p, const SmemTail* tail, int rank) {
-  if (i >= kMaxList) return decode_work<kForm>(w, p, tail, rank);
+  if (i >= kMaxList) return decode_work<kForm, kTo>(w, p, tail, rank);
   const int4 v = tail->list[i];
   constexpr int kStep = Cfg<kForm>::kColStep;
   Work c;
-  c.e = v.x;
+  c.e = v.x & (kWideBit - 1);
+  c.wide = kTo == TO_F16 && v.x >= kWideBit;
   c.nt = v.y;
   c.row0 = v.z;
   c.nrows = v.w;
@@ -236,6 +249,12 @@ __device__ __forceinline__ void cvt_e2m1x8_scaled_f16(uint32_t w, uint32_t sc, u
     out[j] = *reinterpret_cast<const uint32_t*>(&r);
   }
 }
+// (code x scale has at most six significant bits: exact)
+__device__ __forceinline__ uint32_t f16x2_to_bf16x2(uint32_t w) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+  return *reinterpret_cast<const uint32_t*>(&b);
+}
 // Four E4M3 scale bytes -> two f16x2 words (bytes 0,1 and 2,3; low byte -> low half).
 __device__ __forceinline__ void cvt_e4m3x4_f16(uint32_t w, uint32_t& s01, uint32_t& s23) {
   asm("{\n\t.reg .b16 lo, hi;\n\t"
@@ -274,8 +293,7 @@ __device__ __forceinline__ void mma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tme
 
 template <int EPI, int kForm, int kTo>
 __global__ void __launch_bounds__(kThreads, 1)
-grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __grid_constant__ CUtensorMap tmX32,
-                          const __grid_constant__ CUtensorMap tmX16, const __grid_constant__ CUtensorMap tmW,
+grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_constant__ CUtensorMap tmW,
                           const Params p) {
   using C = Cfg<kForm>;
   constexpr bool kPair = C::kPair;
@@ -351,8 +369,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
   const int w_first = kPair ? static_cast<int>(blockIdx.x) >> 1 : static_cast<int>(blockIdx.x);
   const int w_stride = kPair ? static_cast<int>(gridDim.x) >> 1 : static_cast<int>(gridDim.x);
   if (static_cast<int>(threadIdx.x) < kMaxList && w_first + static_cast<int>(threadIdx.x) * w_stride < total_work) {
-    const Work c = decode_work<kForm>(w_first + static_cast<int>(threadIdx.x) * w_stride, p, tail, rank);
-    tail->list[threadIdx.x] = make_int4(c.e, c.nt, c.row0, c.nrows);
+    const Work c = decode_work<kForm, kTo>(w_first + static_cast<int>(threadIdx.x) * w_stride, p, tail, rank);
+    tail->list[threadIdx.x] = make_int4(c.e | (c.wide ? kWideBit : 0), c.nt, c.row0, c.nrows);
   }
   __syncthreads();
   if (kPair) cluster_sync_all();   // both CTAs' barriers are initialised before anyone signals them
@@ -376,7 +394,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       uint32_t rphase = 0;
       bool ok = true;
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kForm>(it, w, p, tail, rank);
+        const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
         const int nt = min(c.nt, p.n_row_tiles - 1);        // half-empty last pair: load the other half again
         const int r0 = p.sub0_base + nt * p.n_step;
         int r1 = p.sub1_base + nt * p.n_step;
@@ -418,17 +436,17 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
     // ------------------------------ token rows (pair: this CTA's half of the columns) ------------
     // a box of 64 or 32 rows and one of 16 (either may be missing) of each k-block of a stage
     if (elect_one()) {
-      tma_prefetch_desc(&tmX64);
-      tma_prefetch_desc(&tmX32);
-      tma_prefetch_desc(&tmX16);
+      for (int i = 0; i < 3; ++i) tma_prefetch_desc(&tmX.m[0][i]);
       int ts = 0;
       uint32_t tphase = 0;
       bool ok = true;
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kForm>(it, w, p, tail, rank);
+        const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
         const int rows = kPair ? c.cols >> 1 : c.cols;       // 16, 32, 48, 64 or 80
         const int big = rows >= 64 ? 64 : (rows & 32);
-        const CUtensorMap* tm = big == 64 ? &tmX64 : &tmX32;
+        const CUtensorMap* maps = tmX.m[c.wide ? 1 : 0];
+        const CUtensorMap* tm = big == 64 ? maps : maps + 1;
+        const CUtensorMap* tm16 = maps + 2;
         const int y = c.row0 + (kPair ? rank * rows : 0);
         for (int kb = 0; kb < p.k_blocks; kb += tok_kbs) {
           if (!mbar_wait_bounded(&tail->tempty[ts], tphase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
@@ -446,8 +464,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
               else tma_load_2d(dst, tm, &tail->tfull[ts], x, y);
             }
             if (rows != big) {
-              if (kPair) tma_load_2d_pair(dst + big * 128, &tmX16, bar, x, y + big);
-              else tma_load_2d(dst + big * 128, &tmX16, &tail->tfull[ts], x, y + big);
+              if (kPair) tma_load_2d_pair(dst + big * 128, tm16, bar, x, y + big);
+              else tma_load_2d(dst + big * 128, tm16, &tail->tfull[ts], x, y + big);
             }
           }
           if (++ts == tok_stages) {
@@ -469,8 +487,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       bool ok = true;
       const uint64_t bdesc0 = make_desc_sw128(smem_u32(sTok));
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kForm>(it, w, p, tail, rank);
-        const uint32_t idesc = make_idesc_16bit(kPair ? 256 : 128, c.cols, kTo != TO_F16);
+        const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
+        const uint32_t idesc = make_idesc_16bit(kPair ? 256 : 128, c.cols, kTo != TO_F16 || c.wide);
         if (!mbar_wait_bounded(&tail->acc_empty[buf], acc_phase[buf] ^ 1, abort_flag, p.status, WAIT_TMEM_EMPTY)) {
           ok = false;
           break;
@@ -545,7 +563,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
     uint32_t raw0 = 0, stage0 = 0;   // raw stages and MMA stages before this tile
     bool ok = true;
     for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-      const Work c = get_work<kForm>(it, w, p, tail, rank);
+      const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
       const int nt = min(c.nt, p.n_row_tiles - 1);
       const int r0 = p.sub0_base + nt * p.n_step;
       int r1 = p.sub1_base + nt * p.n_step;
@@ -555,6 +573,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       const int slot = (row >> 6) * 2 + (wrow >> 7) - (first >> 7);
       const uint32_t sf_off = kSmemCodes + min(slot, 3) * 2048 + (wrow & 31) * 16 + ((wrow >> 5) & 3) * 4;
       // the two groups take the raw stages in turn
+      auto convert = [&](auto as_bf16) {
+      constexpr bool kBf16 = decltype(as_bf16)::value;     // TO_F16: re-encode for an expert marked `wide`
       for (int r = (group + raw0) & 1; r < n_raw; r += kConvGroups) {
         const uint32_t rs = (raw0 + r) % C::kRawStages, rphase = ((raw0 + r) / C::kRawStages) & 1u;
         if (!mbar_wait_bounded(&tail->rfull[rs], rphase, abort_flag, p.status, WAIT_CONVERT)) {
@@ -618,6 +638,10 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
                   out[8 * b + 4 + i] = o1[i];
                 }
               }
+              if (kBf16) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) out[i] = f16x2_to_bf16x2(out[i]);
+              }
               tc_st_32x32b_x16(a_t + 32 * hk + 16 * h, out);
             }
           }
@@ -633,6 +657,9 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
         __syncwarp();
         if (lane == 0) mbar_arrive(&tail->rempty[rs]);
       }
+      };
+      if (kTo == TO_F16 && c.wide) convert(std::true_type{});
+      else convert(std::false_type{});
       raw0 += n_raw;
       stage0 += n_stages;
     }
@@ -644,7 +671,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
     uint32_t acc_phase[2] = {0, 0};
     int buf = 0;
     for (int w = w_first, it = 0; w < total_work; w += w_stride, ++it) {
-      const Work c = get_work<kForm>(it, w, p, tail, rank);
+      const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
       const float alpha = p.alphas[c.e];
       // lane l holds the factors of token t + l of the warp's next 32 (FC2: 16) columns; the first are
       // fetched before the accumulator is waited for
@@ -652,7 +679,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       auto row_of = [&](int t) {
         return c.row0 + min(t + (EPI == EPI_FC2 ? (lane & 15) : lane), c.nrows - 1);
       };
-      float inv_next = kTo == TO_F16 ? p.row_inv[row_of(t_first)] : 1.0f;
+      auto inv_of = [&](int t) { return c.wide ? 1.0f : p.row_inv[row_of(t)]; };
+      float inv_next = kTo == TO_F16 ? inv_of(t_first) : 1.0f;
       if (!mbar_wait_idle(&tail->acc_full[buf], acc_phase[buf], abort_flag, p.status, WAIT_TMEM_FULL)) break;
       acc_phase[buf] ^= 1;
       tc_fence_after();
@@ -666,7 +694,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
           tc_ld_32x32b_x16(t_lane + ch, r);
           tc_wait_ld();
           const float inv_l = inv_next;
-          if (kTo == TO_F16 && ch + 32 < c.cols) inv_next = p.row_inv[row_of(ch + 32)];
+          if (kTo == TO_F16 && ch + 32 < c.cols) inv_next = inv_of(ch + 32);
           float* o = p.out_f32 + static_cast<size_t>(c.row0 + ch) * p.out_cols + col;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -678,7 +706,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __gri
       } else {
         for (int t0 = 32 * half; t0 < c.cols; t0 += 64) {
           const float inv_l = inv_next;
-          if (kTo == TO_F16 && t0 + 64 < c.cols) inv_next = p.row_inv[row_of(t0 + 64)];
+          if (kTo == TO_F16 && t0 + 64 < c.cols) inv_next = inv_of(t0 + 64);
           const float al_l = p.route_weights != nullptr
                                  ? __fmul_rn(alpha, p.route_weights[p.sorted_route_ids[row_of(t0)]]) : alpha;
 #pragma unroll
@@ -834,13 +862,15 @@ __global__ void __launch_bounds__(256) permute_rows_bf16_kernel(
 
 // The same, and the rows once more as FP16 (rows_bf16 and sorted_route_ids null: rows that lie in sorted order
 // already, FC2's, as FP16 only), each multiplied by the power of two that puts its largest finite magnitude
-// into [2^14, 2^15); row_inv[pos] takes the inverse.  BF16 has 8 significant bits: every value down
-// to 2^-32 of the row's largest is carried over exactly, anything smaller to within 2^-40 of it,
-// far below one rounding of the FP32 accumulator.  Infinities and NaNs stay what they are.
+// into [2^14, 2^15); row_inv[pos] takes the inverse.  BF16 has 8 significant bits: every value down to 2^-31
+// of the row's largest binade is carried over exactly.  A row with smaller ones marks its expert `wide`
+// (a mark too many is still right: such an expert's GEMMs run on the BF16 rows, at a lower rate; the sort clears
+// the marks).  Infinities and NaNs stay what they are.
 __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* __restrict__ expert_offsets,
     int E, const int32_t* __restrict__ sorted_route_ids, int num_topk, int K,
-    __nv_bfloat16* __restrict__ rows_bf16, __half* __restrict__ out, float* __restrict__ row_inv) {
+    __nv_bfloat16* __restrict__ rows_bf16, __half* __restrict__ out, float* __restrict__ row_inv,
+    int32_t* __restrict__ wide) {
   const int total = expert_offsets[E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = K >> 3;
@@ -849,12 +879,17 @@ __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(tkn) * x_row_stride);
     uint4* copy = rows_bf16 != nullptr ? reinterpret_cast<uint4*>(rows_bf16 + static_cast<size_t>(pos) * K) : nullptr;
     __nv_bfloat162 m2 = __float2bfloat162_rn(0.f);
+    // smallest nonzero magnitude: + 0x7fff takes 0 to the largest signed 16-bit value and keeps the others in order
+    uint32_t least2 = 0x7fff7fffu;
     for (int j = lane; j < nvec; j += 32) {
       const uint4 v = __ldg(src + j);
       if (copy != nullptr) copy[j] = v;
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+      for (int i = 0; i < 4; ++i) {
+        m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+        least2 = __vmins2(least2, (w[i] & 0x7fff7fffu) + 0x7fff7fffu);
+      }
     }
     // BF16 magnitudes order like their bits
     uint32_t m = __reduce_max_sync(0xffffffffu, static_cast<uint32_t>(max(__bfloat16_as_ushort(__low2bfloat16(m2)),
@@ -876,7 +911,20 @@ __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
     // exponent field e of the largest: x 2^(141 - e), the factor kept a normal float either way
     const int sh = min(141 - max(static_cast<int>(m >> 7), 1), 126);
     const float scale = __uint_as_float(static_cast<uint32_t>(127 + sh) << 23);
-    if (lane == 0) row_inv[pos] = __uint_as_float(static_cast<uint32_t>(127 - sh) << 23);
+    // the last bit of a value with exponent field f is 2^(f - 134 + sh) of the FP16 row, whose last is 2^-24
+    const int least = __reduce_min_sync(0xffffffffu, min(static_cast<int>(static_cast<int16_t>(least2 & 0xffffu)),
+                                                         static_cast<int>(least2) >> 16)) + 0x8001;
+    if (lane == 0) {
+      row_inv[pos] = __uint_as_float(static_cast<uint32_t>(127 - sh) << 23);
+      if (max(least >> 7, 1) + sh < 110) {
+        int lo = 0, hi = E - 1;      // the expert of the row: the last whose first row is not behind it
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (expert_offsets[mid] <= pos) lo = mid; else hi = mid - 1;
+        }
+        wide[lo] = 1;
+      }
+    }
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(pos) * K);
     for (int j = lane; j < nvec; j += 32) {
       const uint4 v = __ldg(src + j);
@@ -926,7 +974,7 @@ static int make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t cols, uin
 }
 
 template <int EPI, int kForm, int kTo>
-static int launch(const CUtensorMap (&tmX)[3], const CUtensorMap& tmW, const Params& p, int ctas, cudaStream_t s) {
+static int launch(const TokenMaps& tmX, const CUtensorMap& tmW, const Params& p, int ctas, cudaStream_t s) {
   constexpr bool kPair = Cfg<kForm>::kPair;
   auto kern = grouped_gemm_w4a16_kernel<EPI, kForm, kTo>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<kForm>()) != cudaSuccess)
@@ -949,7 +997,7 @@ static int launch(const CUtensorMap (&tmX)[3], const CUtensorMap& tmW, const Par
     if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) return B200MOE_ECUDA;
     if (2 * clusters < static_cast<int>(cfg.gridDim.x)) cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
   }
-  return cudaLaunchKernelEx(&cfg, kern, tmX[0], tmX[1], tmX[2], tmW, p) == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
+  return cudaLaunchKernelEx(&cfg, kern, tmX, tmW, p) == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }
 
 // One CTA up to 18 rows per expert (finer tiles, no partner to wait for), narrow pairs to 58 (nearly every
@@ -970,12 +1018,14 @@ static int form_for(const b200moe_gemm_args* a) {
 }
 
 template <int EPI, int kTo>
-static int launch_any(const b200moe_gemm_args* a, const void* tokens, uint64_t cols, const void* weights, Params& p,
-                      cudaStream_t s) {
-  CUtensorMap tmX[3], tmW;
+static int launch_any(const b200moe_gemm_args* a, const void* tokens, const void* tokens_bf16, uint64_t cols,
+                      const void* weights, Params& p, cudaStream_t s) {
+  TokenMaps tmX;
+  CUtensorMap tmW;
   const uint32_t boxes[3] = {64, 32, 16};
   for (int i = 0; i < 3; ++i) {
-    const int rc = make_tmap_bf16(&tmX[i], tokens, cols, a->layout->rows, boxes[i]);
+    int rc = make_tmap_bf16(&tmX.m[0][i], tokens, cols, a->layout->rows, boxes[i]);
+    if (rc == B200MOE_OK) rc = make_tmap_bf16(&tmX.m[1][i], tokens_bf16, cols, a->layout->rows, boxes[i]);
     if (rc != B200MOE_OK) return rc;
   }
   const int rc = make_tmap_bytes_2d(&tmW, weights, cols / 2, static_cast<uint64_t>(a->num_experts) * p.w_rows, 64);
@@ -992,6 +1042,11 @@ static int launch_any(const b200moe_gemm_args* a, const void* tokens, uint64_t c
 static int row_grid(int rows) {
   const int ctas = (rows + 7) / 8;
   return ctas < 148 * 8 ? ctas : 148 * 8;
+}
+
+// [2][E]: FC1's and FC2's marks, behind the expert counts
+static int32_t* wide_marks(const b200moe_gemm_args* a, char* base) {
+  return reinterpret_cast<int32_t*>(base + a->layout->expert_counts) + a->num_experts;
 }
 
 static void fill_common(Params& p, const b200moe_gemm_args* a, char* base) {
@@ -1023,11 +1078,12 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
   const bool f16 = !a->sf_e8m0;
   const int32_t* offsets = reinterpret_cast<const int32_t*>(base + L.expert_offsets);
   const int32_t* routes = reinterpret_cast<const int32_t*>(base + L.sorted_route_ids);
+  int32_t* wide = wide_marks(a, base);
   if (f16)
     permute_rows_f16_kernel<<<ggrid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes, a->num_topk, K,
         reinterpret_cast<__nv_bfloat16*>(base + L.act_q), reinterpret_cast<__half*>(base + L.mid_sf),
-        reinterpret_cast<float*>(base + L.act_sf));
+        reinterpret_cast<float*>(base + L.act_sf), wide);
   else
     permute_rows_bf16_kernel<<<ggrid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes, a->num_topk, K,
@@ -1039,6 +1095,7 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
   p.alphas = a->w1_alphas;
   p.out_bf16 = reinterpret_cast<__nv_bfloat16*>(base + L.mid_q);
   p.row_inv = reinterpret_cast<const float*>(base + L.act_sf);
+  p.wide = wide;
   p.tap = a->fc1_tap;
   p.route_weights = a->fc1_route_weights;
   p.sorted_route_ids = reinterpret_cast<const int32_t*>(base + L.sorted_route_ids);
@@ -1053,15 +1110,15 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
     p.n_step = 64;
     p.sub0_base = a->gate_first ? I : 0;   // up rows
     p.sub1_base = a->gate_first ? 0 : I;   // gate rows
-    return f16 ? launch_any<EPI_FC1_GATED, TO_F16>(a, tokens, K, a->w13, p, stream)
-               : launch_any<EPI_FC1_GATED, TO_BF16_E8M0>(a, tokens, K, a->w13, p, stream);
+    return f16 ? launch_any<EPI_FC1_GATED, TO_F16>(a, tokens, base + L.act_q, K, a->w13, p, stream)
+               : launch_any<EPI_FC1_GATED, TO_BF16_E8M0>(a, tokens, base + L.act_q, K, a->w13, p, stream);
   }
   p.n_row_tiles = ceil_div_i(I, 128);
   p.n_step = 128;
   p.sub0_base = 0;
   p.sub1_base = 64;
-  return f16 ? launch_any<EPI_FC1_RELU2, TO_F16>(a, tokens, K, a->w13, p, stream)
-             : launch_any<EPI_FC1_RELU2, TO_BF16_E8M0>(a, tokens, K, a->w13, p, stream);
+  return f16 ? launch_any<EPI_FC1_RELU2, TO_F16>(a, tokens, base + L.act_q, K, a->w13, p, stream)
+             : launch_any<EPI_FC1_RELU2, TO_BF16_E8M0>(a, tokens, base + L.act_q, K, a->w13, p, stream);
 }
 
 int w4a16_gemm2(const b200moe_gemm_args* a, cudaStream_t stream) {
@@ -1085,15 +1142,17 @@ int w4a16_gemm2(const b200moe_gemm_args* a, cudaStream_t stream) {
   p.n_step = 128;
   p.sub0_base = 0;
   p.sub1_base = 64;
-  if (a->sf_e8m0) return launch_any<EPI_FC2, TO_BF16_E8M0>(a, base + L.mid_q, I, a->w2, p, stream);
+  if (a->sf_e8m0) return launch_any<EPI_FC2, TO_BF16_E8M0>(a, base + L.mid_q, base + L.mid_q, I, a->w2, p, stream);
   // the intermediate rows as FP16, in the place of FC1's
   const int rows = a->num_tokens * a->num_topk;
   float* row_inv = reinterpret_cast<float*>(base + L.act_sf) + L.rows;
+  int32_t* wide = wide_marks(a, base) + E;
   permute_rows_f16_kernel<<<row_grid(rows), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(base + L.mid_q), I, p.expert_offsets, E, nullptr, 1, I, nullptr,
-      reinterpret_cast<__half*>(base + L.mid_sf), row_inv);
+      reinterpret_cast<__half*>(base + L.mid_sf), row_inv, wide);
   p.row_inv = row_inv;
-  return launch_any<EPI_FC2, TO_F16>(a, base + L.mid_sf, I, a->w2, p, stream);
+  p.wide = wide;
+  return launch_any<EPI_FC2, TO_F16>(a, base + L.mid_sf, base + L.mid_q, I, a->w2, p, stream);
 }
 
 int w4a16_activation_amax(const b200moe_amax_args* a, cudaStream_t stream) {

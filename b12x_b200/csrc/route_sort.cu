@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kSortThreads) expert_sort_kernel(
     int32_t* __restrict__ tile_base, int32_t* __restrict__ mtile_expert,
     int32_t* __restrict__ mtile_row0, int32_t* __restrict__ mtile_rows,
     int32_t* __restrict__ sorted_route_ids, int32_t* __restrict__ inv_perm, int mtile_cap,
-    int tile_rows, int count_warps, const int32_t* wait_flags, const int32_t* wait_epoch_dev, int32_t* wait_status,
+    int tile_rows, int count_warps, int32_t* __restrict__ marks, const int32_t* wait_flags, const int32_t* wait_epoch_dev, int32_t* wait_status,
     int wait_world, unsigned long long wait_limit_ns) {
   extern __shared__ int32_t smem[];
   if (wait_flags != nullptr) {
@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kSortThreads) expert_sort_kernel(
     tile_base[e] = tbase[e];
     if (e < E) {
       expert_counts[e] = etotal[e];
+      if (marks != nullptr) marks[e] = marks[E + e] = 0;
       const int nt = (etotal[e] + tile_rows - 1) >> tile_shift;
       for (int t = 0; t < nt; ++t) {
         const int mt = tbase[e] + t;
@@ -251,7 +252,8 @@ __global__ void __launch_bounds__(kChunkThreads) sort_count_kernel(
 __global__ void __launch_bounds__(1024) sort_scan_kernel(
     int chunks, int E, int32_t* __restrict__ chunk_counts, int32_t* __restrict__ expert_counts,
     int32_t* __restrict__ expert_offsets, int32_t* __restrict__ tile_base, int32_t* __restrict__ mtile_expert,
-    int32_t* __restrict__ mtile_row0, int32_t* __restrict__ mtile_rows, int mtile_cap, int tile_rows) {
+    int32_t* __restrict__ mtile_row0, int32_t* __restrict__ mtile_rows, int mtile_cap, int tile_rows,
+    int32_t* __restrict__ marks) {
   extern __shared__ int32_t smem[];
   int32_t* etotal = smem;             // [E]
   int32_t* eoffs = etotal + E;        // [E+1]
@@ -303,7 +305,10 @@ __global__ void __launch_bounds__(1024) sort_scan_kernel(
   for (int e = threadIdx.x; e <= E; e += blockDim.x) {
     expert_offsets[e] = eoffs[e];
     tile_base[e] = tbase[e];
-    if (e < E) expert_counts[e] = etotal[e];
+    if (e < E) {
+      expert_counts[e] = etotal[e];
+      marks[e] = marks[E + e] = 0;
+    }
   }
   // row tiles: one warp per expert at a time (an expert of a large batch has many tiles)
   for (int e = warp; e < E; e += (blockDim.x >> 5)) {
@@ -408,6 +413,7 @@ extern "C" int b200moe_expert_sort(const b200moe_sort_args* a, void* stream) {
     return B200MOE_EINVAL;
   if (rows > L.rows) return B200MOE_ECAPACITY;
   char* base = static_cast<char*>(a->scratch);
+  int32_t* marks = reinterpret_cast<int32_t*>(base + L.expert_counts) + E;    // per expert and GEMM, see the layout
   const unsigned long long limit_ns =
       a->wait_timeout_ms > 0 ? static_cast<unsigned long long>(a->wait_timeout_ms) * 1000000ull : kWaitLimitNs;
   if (rows >= kMultiCtaSortRows) {
@@ -422,7 +428,7 @@ extern "C" int b200moe_expert_sort(const b200moe_sort_args* a, void* stream) {
         chunks, E, chunk_counts, reinterpret_cast<int32_t*>(base + L.expert_counts),
         reinterpret_cast<int32_t*>(base + L.expert_offsets), reinterpret_cast<int32_t*>(base + L.tile_base),
         reinterpret_cast<int32_t*>(base + L.mtile_expert), reinterpret_cast<int32_t*>(base + L.mtile_row0),
-        reinterpret_cast<int32_t*>(base + L.mtile_rows), L.mtile_cap, L.tile_rows == 64 ? 64 : 128);
+        reinterpret_cast<int32_t*>(base + L.mtile_rows), L.mtile_cap, L.tile_rows == 64 ? 64 : 128, marks);
     sort_scatter_kernel<<<chunks, kChunkThreads, static_cast<size_t>(kChunkThreads / 32) * E * 4, s>>>(
         a->topk_ids, a->expert_map, a->expert_map_len, rows, E, chunk_counts,
         reinterpret_cast<const int32_t*>(base + L.expert_offsets), reinterpret_cast<int32_t*>(base + L.sorted_route_ids),
@@ -448,7 +454,7 @@ extern "C" int b200moe_expert_sort(const b200moe_sort_args* a, void* stream) {
       reinterpret_cast<int32_t*>(base + L.mtile_rows),
       reinterpret_cast<int32_t*>(base + L.sorted_route_ids),
       reinterpret_cast<int32_t*>(base + L.inv_perm), L.mtile_cap,
-      L.tile_rows == 64 ? 64 : 128, nwarps, a->wait_flags, a->wait_epoch_dev, a->wait_status, a->wait_world, limit_ns);
+      L.tile_rows == 64 ? 64 : 128, nwarps, marks, a->wait_flags, a->wait_epoch_dev, a->wait_status, a->wait_world, limit_ns);
   return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }
 
@@ -525,6 +531,6 @@ extern "C" int b200moe_expert_sort_static(const int32_t* topk_ids, const int32_t
       topk_ids, expert_map, expert_map_len, rows, num_experts, w + kStaticOffStatus,
       w + kStaticOffCounts, expert_offsets, w + kStaticOffTileBase, w + kStaticOffMtileExpert,
       w + kStaticOffMtileRow0, w + kStaticOffMtileRows, sorted_route_ids, inv_perm,
-      kStaticSortMtileCap, 128, nwarps, nullptr, nullptr, nullptr, 0, 0ull);
+      kStaticSortMtileCap, 128, nwarps, nullptr, nullptr, nullptr, nullptr, 0, 0ull);
   return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }

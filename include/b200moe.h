@@ -69,7 +69,8 @@ typedef struct {
 typedef struct {
   int64_t total_nbytes;
   int64_t status;            /* int32[16]; word 0: device error, word 1: where  */
-  int64_t expert_counts;     /* int32[E]                                        */
+  int64_t expert_counts;     /* int32[E]; behind it int32[2][E], cleared by the sort: w4a16 marks of experts whose
+                                FC1 / FC2 rows go into the MMA as BF16, not FP16 */
   int64_t expert_offsets;    /* int32[E+1]  first sorted position per expert    */
   int64_t tile_base;         /* int32[E+1]  first row tile per expert           */
   int64_t mtile_expert;      /* int32[mtile_cap]                                */

@@ -100,3 +100,54 @@ def test_token_rows_are_readable_after_a_run(tokens, hidden, inter):
         for which, v in enumerate((x.float(), mid)):
             part = v[offs[e]:offs[e + 1]].abs()
             assert amax[0, e, which].item() == (part.max().item() if part.numel() else 0.0)
+
+
+def _rowwise(got, ref, tol):
+    """Row by row, since the rows' sizes lie far apart: max-abs error <= tol x the row's RMS."""
+    err = (got - ref).abs().amax(dim=1)
+    rms = ref.double().square().mean(dim=1).sqrt().float()
+    assert bool((rms > 0).all()) and bool((err <= tol * rms).all()), (err / rms).max()
+
+
+@pytest.mark.parametrize("tokens,experts,act", [(40, 4, "silu"), (40, 2, "silu"), (140, 2, "silu"), (40, 4, "relu2"),
+                                                (140, 2, "relu2")])
+def test_rows_wider_than_fp16(tokens, experts, act):
+    """Rows whose largest element lies 20 to 60 binades above the others and meets a zero weight, so that the small
+    elements are the whole sum: up to 31 binades on FP16 operands (expert 0), beyond on BF16 operands."""
+    shp = _w16(tokens=tokens, experts=experts, topk=1, hidden=320, intermediate=192, activation=act)
+    inp = synth.make_inputs(shp, seed=tokens)
+    gap = 20 + torch.arange(tokens) * 41 // tokens
+    gen = torch.Generator().manual_seed(3)
+    x = (torch.rand(tokens, 320, generator=gen) * 1.5 + 0.5) * (torch.randint(0, 2, (tokens, 320), generator=gen) * 2 - 1)
+    x *= torch.exp2(17.0 - gap)[:, None]
+    x[:, 0] = 2.0 ** 17                                 # 2 ** (gap + 1) above the smallest
+    w1 = inp.w1_fp4.clone()
+    w1[..., 0] &= 0xF0                                  # the weights of element 0
+    inp = replace(inp, x=x.to(torch.bfloat16), w1_fp4=w1)
+    ids = (gap > 30).to(torch.int32).reshape(-1, 1)
+    run = run_layer(inp, topk_ids=ids, topk_weights=torch.ones(tokens, 1))
+    _, taps = oracle_layer(inp, ids, torch.ones(tokens, 1))
+    _rowwise(run.fc1[:tokens], taps.fc1, 1e-4)          # fp32 sums of 320 terms in another order
+
+
+@pytest.mark.parametrize("tokens,experts", [(30, 4), (40, 2), (140, 2)])
+def test_intermediate_rows_wider_than_fp16(tokens, experts):
+    """The same for FC2: 16 intermediate columns 2 ** 36 above the others, with zero weights in FC2."""
+    shp = _w16(tokens=tokens, experts=experts, topk=1, hidden=64, intermediate=192)
+    inp = synth.make_inputs(shp, seed=tokens)
+    gen = torch.Generator().manual_seed(4)
+    x = (torch.rand(tokens, 64, generator=gen) * 0.5 + 0.5).to(torch.bfloat16)
+    codes = torch.randint(1, 8, (experts, 384, 64), generator=gen).to(torch.uint8)          # positive weights
+    scale = torch.full((384, 4), 0x01, dtype=torch.uint8)                                   # 2 ** -9 ...
+    scale[:16] = scale[192:208] = 0x7E                                                      # ... and 448
+    w2 = inp.w2_fp4.clone()
+    w2[..., :8] = 0
+    inp = replace(inp, x=x, w1_fp4=codes[..., 0::2] | codes[..., 1::2] << 4, w2_fp4=w2,
+                  w1_blockscale=synth.swizzle_block_scale(scale).expand(experts, -1, -1).contiguous().view(inp.w1_blockscale.dtype),
+                  w1_global_scale=torch.ones_like(inp.w1_global_scale))
+    ids = torch.ones(tokens, 1, dtype=torch.int32)
+    run = run_layer(inp, topk_ids=ids, topk_weights=torch.ones(tokens, 1))
+    _, taps = oracle_layer(inp, ids, torch.ones(tokens, 1))
+    mid = taps.mid.abs()
+    assert (mid.amax(dim=1) / mid.amin(dim=1)).min() > 2.0 ** 34
+    _rowwise(run.out_f32, taps.out_f32, 1e-2)           # BF16 roundings of the intermediate that fall the other way
