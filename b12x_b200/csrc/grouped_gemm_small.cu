@@ -399,6 +399,7 @@ grouped_gemm_small_kernel(const __grid_constant__ CUtensorMap tmW,
           ok = false;
           break;
         }
+        tc_fence_after();          // behind the MMAs that read these columns (the producer waited for them)
         const uint8_t* sf = sSf + stage * 3 * kSmemSf;
         const uint4 a = reinterpret_cast<const uint4*>(sf)[lane];
         const uint4 b = reinterpret_cast<const uint4*>(sf + kSmemSf)[lane];
