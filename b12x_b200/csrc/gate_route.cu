@@ -13,6 +13,8 @@
 // product written in the operands' common type, then the bias added in that type): fp32
 // accumulation, one rounding to bf16 when both operands are bf16, the bias added with one more
 // rounding.  The router then works on the stored logits (same routine as b200moe_route_topk).
+#include <type_traits>
+
 #include "cluster_pair.cuh"
 #include "gemm_shared.cuh"
 #include "route_shared.cuh"
@@ -156,13 +158,20 @@ __global__ void __launch_bounds__(256) gate_route_simt_kernel(b200moe_gate_route
 // 3.7 MB at 256 x 7168, which one SM takes some 35 us to bring in from L2), and a batch has few
 // tiles, so a CLUSTER of up to eight CTAs shares one: each multiplies its part of K into its own
 // TMEM accumulator, leaves the fp32 partial sums in shared memory, and after a cluster barrier
-// sums the parts of 128 / S of the tokens out of the S shared memories, in order of S, rounds
-// them and routes those tokens, one warp per token.  4096 tokens x 256 experts, K 7168: 332 us with
-// one CTA per tile (32 SMs, each of four warps routing 32 tokens), 40 us now (28 us with the
-// operands in L2); what is left is the operands' way into each SM and the routing at the end.
+// sums the parts of 128 / S of the tokens out of the S shared memories, rounds them and routes
+// those tokens, one warp per token.  4096 tokens x 256 experts, K 7168: 332 us with one CTA per tile
+// (32 SMs, each of four warps routing 32 tokens), 37 us now (27 us with the operands in L2); what is
+// left is the operands' way into each SM and the routing at the end.
+//
+// A token's logits do not depend on the batch it comes in: K is cut into as many parts (a power of
+// two, eight where K has eight k-blocks) whatever the number of tokens, and the parts are summed
+// pairwise, (0+1)+(2+3)+..., in every batch.  Where clusters of that many CTAs exceed the SMs, a CTA
+// takes two, four or eight neighbouring parts, each in a TMEM accumulator of its own, as far as the 512
+// columns go (256 experts: two).  Against cutting K by the number of tokens this costs batches of more than
+// 4736 tokens x 256 experts (8192: 51 -> 59 us, 16384: 93 -> 116 us), nothing elsewhere.
 constexpr int kTcThreads = 512;       // TMA warp, MMA warp, four epilogue warps; all sixteen warps route
 constexpr int kTcStages = 4;
-constexpr int kTcMaxSplit = 8;        // portable cluster size
+constexpr int kTcLogSplit = 3;        // eight parts: the portable cluster size
 struct __align__(8) GateTail {
   uint64_t full[kTcStages];
   uint64_t empty[kTcStages];
@@ -171,15 +180,53 @@ struct __align__(8) GateTail {
   int abort_flag;
 };
 
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
+}
+
+// Pairwise sum over the S CTAs of the cluster of the four partial sums at `src`.  All loads are under way
+// before the first sum, four values each: one value at a time, part after part, takes 17 instead of 16 us at 64
+// tokens x 256 experts and 20 instead of 17 us at 512.
+template <int S>
+__device__ __forceinline__ float4 sum_splits(uint32_t src) {
+  float4 v[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) v[s] = ld_cluster_f32x4(pair::map_to_cta(src, static_cast<uint32_t>(s)));
+#pragma unroll
+  for (int w = 1; w < S; w <<= 1) {
+#pragma unroll
+    for (int s = 0; s < S; s += 2 * w) {
+      v[s].x = __fadd_rn(v[s].x, v[s + w].x);
+      v[s].y = __fadd_rn(v[s].y, v[s + w].y);
+      v[s].z = __fadd_rn(v[s].z, v[s + w].z);
+      v[s].w = __fadd_rn(v[s].w, v[s + w].w);
+    }
+  }
+  return v[0];
+}
+
+// v[i] = pairwise sum over N neighbouring accumulators of `cols` TMEM columns each
+template <int N>
+__device__ __forceinline__ void ld_accumulators(uint32_t taddr, int cols, uint32_t (&v)[16]) {
+  if constexpr (N == 1) {
+    tc_ld_32x32b_x16(taddr, v);
+    tc_wait_ld();
+  } else {
+    uint32_t hi[16];
+    ld_accumulators<N / 2>(taddr, cols, v);
+    ld_accumulators<N / 2>(taddr + N / 2 * cols, cols, hi);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      v[i] = __float_as_uint(__fadd_rn(__uint_as_float(v[i]), __uint_as_float(hi[i])));
+  }
 }
 
 __global__ void __launch_bounds__(kTcThreads, 1)
 gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-                     b200moe_gate_route_args g, b200moe_route_args r, int tmem_cols, int splits) {
+                     b200moe_gate_route_args g, b200moe_route_args r, int acc_cols, int log_parts, int splits) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -196,7 +243,10 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_blocks = (K + 63) / 64;                // 64 bf16 = one 128-byte swizzled row
   const int rank = static_cast<int>(pair::cluster_ctarank());
-  const int kb0 = k_blocks * rank / splits, kb1 = k_blocks * (rank + 1) / splits;
+  // this CTA's parts of the reduction, each with an accumulator of its own
+  const int per_cta = (1 << log_parts) / splits, part0 = rank * per_cta;
+  const int tmem_cols = acc_cols * per_cta;
+  const int kb0 = k_blocks * part0 >> log_parts, kb1 = k_blocks * (part0 + per_cta) >> log_parts;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTcStages; ++s) {
@@ -254,7 +304,15 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int part = part0, kb_part = kb0;              // k-blocks before the current part and
+      int kb_next = k_blocks * (part + 1) >> log_parts;   // ... before the next
       for (int kb = kb0; kb < kb1; ++kb) {
+        if (kb == kb_next) {
+          ++part;
+          kb_part = kb;
+          kb_next = k_blocks * (part + 1) >> log_parts;
+        }
+        const uint32_t d_tmem = tmem_base + (part - part0) * acc_cols;
         if (!mbar_wait_bounded(&tail->full[stage], phase, abort_flag, g.status, WAIT_SMEM_FULL)) {
           ok = false;
           break;
@@ -265,7 +323,7 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         // four MMAs of 16 elements; the zero-filled tail of the last k-block adds nothing
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          mma_bf16(tmem_base, adesc + 2 * j, bdesc + 2 * j, idesc, (kb > kb0 || j > 0) ? 1u : 0u);
+          mma_bf16(d_tmem, adesc + 2 * j, bdesc + 2 * j, idesc, (kb > kb_part || j > 0) ? 1u : 0u);
         tc_commit(&tail->empty[stage]);
         if (++stage == kTcStages) {
           stage = 0;
@@ -282,14 +340,19 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       tc_fence_after();
       const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(sub * 32) << 16);
       float* row = sPart + (sub * 32 + lane) * part_stride;
-      for (int c = 0; c < E; c += 16) {
-        uint32_t v[16];
-        tc_ld_32x32b_x16(t_lane + c, v);
-        tc_wait_ld();
+      auto drain = [&](auto count) {
+        for (int c = 0; c < E; c += 16) {
+          uint32_t v[16];
+          ld_accumulators<decltype(count)::value>(t_lane + c, acc_cols, v);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(row + c + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      }
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(row + c + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+      };
+      if (per_cta == 1) drain(std::integral_constant<int, 1>{});
+      else if (per_cta == 2) drain(std::integral_constant<int, 2>{});
+      else if (per_cta == 4) drain(std::integral_constant<int, 4>{});
+      else drain(std::integral_constant<int, 8>{});
     }
   }
   tc_fence_before();
@@ -306,23 +369,17 @@ gate_route_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     const int row = rank * share + i;
     const int t = t0 + row;
     if (t >= T) break;
-    float acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int s = 0; s < splits; ++s) {
-      const uint32_t src = pair::map_to_cta(part_addr, static_cast<uint32_t>(s)) +
-                           static_cast<uint32_t>(row * part_stride) * 4u;
-      float v[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = j * 32 + lane < E ? ld_cluster_f32(src + (j * 32 + lane) * 4) : 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], v[j]);
-    }
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.logits_out) + static_cast<int64_t>(t) * E;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int e = j * 32 + lane;
-      if (e < E) out[e] = __float2bfloat16_rn(finish_logit(acc[j], g.gate_bias, e, g.bias_dtype, true));
+    for (int e = 4 * lane; e < E; e += 128) {
+      const uint32_t src = part_addr + static_cast<uint32_t>(row * part_stride + e) * 4u;
+      const float4 a = splits == 8 ? sum_splits<8>(src) : splits == 4 ? sum_splits<4>(src)
+                       : splits == 2 ? sum_splits<2>(src) : sum_splits<1>(src);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(finish_logit(a.x, g.gate_bias, e, g.bias_dtype, true),
+                                                      finish_logit(a.y, g.gate_bias, e + 1, g.bias_dtype, true));
+      const __nv_bfloat162 hi = __floats2bfloat162_rn(finish_logit(a.z, g.gate_bias, e + 2, g.bias_dtype, true),
+                                                      finish_logit(a.w, g.gate_bias, e + 3, g.bias_dtype, true));
+      *reinterpret_cast<uint2*>(out + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
+                                                      *reinterpret_cast<const uint32_t*>(&hi));
     }
     __syncwarp();                // the row is in global memory for the lane that reads the winner's logit
     route_token_any<8>(r, t, lane);
@@ -409,13 +466,19 @@ extern "C" int b200moe_gate_route(const b200moe_gate_route_args* g, void* stream
     if (rc != B200MOE_OK) return rc;
     int cols = 32;
     while (cols < E) cols <<= 1;
-    const int smem = 1024 + kTcStages * (16384 + ((E * 128 + 1023) & ~1023)) + static_cast<int>(sizeof(GateTail));
+    // At least 116 KB, so that an SM holds one CTA: with two, CTAs of two clusters could wait for each other's
+    // tensor memory (an allocation waits until the columns are free) across a cluster barrier.
+    const int smem_ring = 1024 + kTcStages * (16384 + ((E * 128 + 1023) & ~1023)) + static_cast<int>(sizeof(GateTail));
+    const int smem = smem_ring < 116 * 1024 ? 116 * 1024 : smem_ring;
     if (cudaFuncSetAttribute(gate_route_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return B200MOE_ECUDA;
-    // as many parts of the reduction per token tile as keep all SMs busy, each with a k-block or more
+    // parts of the reduction by K alone; one per CTA where that keeps to the SMs, else more
     const int tiles = (T + 127) / 128, k_blocks = (K + 63) / 64, sms = num_sms_cached();
-    int splits = kTcMaxSplit;
-    while (splits > 1 && (tiles * splits > sms || splits > k_blocks)) splits >>= 1;
+    int log_parts = kTcLogSplit;
+    while ((1 << log_parts) > k_blocks) --log_parts;
+    const int parts = 1 << log_parts;
+    int splits = parts;
+    while (splits > 1 && tiles * splits > sms && parts / splits * 2 * cols <= 512) splits >>= 1;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -428,7 +491,7 @@ extern "C" int b200moe_gate_route(const b200moe_gate_route_args* g, void* stream
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gate_route_tc_kernel, tmX, tmW, *g, r, cols, splits) == cudaSuccess
+    return cudaLaunchKernelEx(&cfg, gate_route_tc_kernel, tmX, tmW, *g, r, cols, log_parts, splits) == cudaSuccess
                ? B200MOE_OK : B200MOE_ECUDA;
   }
   if (kernel != B200MOE_GATE_SIMT) return B200MOE_EINVAL;

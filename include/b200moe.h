@@ -128,8 +128,9 @@ int b200moe_route_topk(const b200moe_route_args* a, void* stream);
  * (fp32 accumulation; one rounding for the product, one more for the bias).
  * The router then runs on the stored logits with the semantics of
  * b200moe_route_topk.  `kernel` picks the implementation: AUTO = tensor cores for
- * bf16 operands with E % 16 == 0, E <= 256, K % 8 == 0 and at least 128 tokens,
- * else the CUDA-core kernel. */
+ * bf16 operands with E % 16 == 0, E <= 256, K % 8 == 0, 16-byte aligned rows and at
+ * least 128 tokens or E * K >= 32768, else the CUDA-core kernel.  On the tensor cores
+ * a token's logits do not depend on the number of tokens in the call. */
 enum { B200MOE_GATE_AUTO = 0, B200MOE_GATE_SIMT = 1, B200MOE_GATE_TC = 2 };
 typedef struct {
   const void* hidden;        /* [T][hidden_row_stride] bf16 or f32                */

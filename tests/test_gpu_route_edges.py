@@ -83,3 +83,19 @@ def test_split_gate_kernel(tokens, hidden, experts, topk):
     _, ids, w = O.route_topk(got, topk)
     assert torch.equal(r.topk_ids.cpu(), ids)
     torch.testing.assert_close(r.topk_weights.cpu(), w, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("hidden,experts", [(1096, 256), (2048, 32), (320, 64)])     # 18, 32 and 5 k-blocks
+def test_logits_do_not_depend_on_the_batch(hidden, experts):
+    """K is cut and summed alike for every number of tokens, whatever the number of CTAs that share a tile."""
+    gen = torch.Generator().manual_seed(hidden)
+    hs = torch.randn(9700, hidden, generator=gen).to(torch.bfloat16).to(DEV)
+    gw = (torch.randn(experts, hidden, generator=gen) * 0.05).to(torch.bfloat16).to(DEV)
+
+    def logits(n):
+        return fused_moe.route(binding=fused_moe.bind_route(hidden_states=hs[:n], top_k=2, gate_weight=gw,
+                                                            gate_kernel="tc")).router_logits
+
+    whole = logits(9700)
+    for n in (1, 100, 2304, 2433, 4736, 4737):
+        assert torch.equal(logits(n), whole[:n]), n
