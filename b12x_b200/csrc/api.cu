@@ -10,7 +10,7 @@ bool nvfp4_small_batch_ok(const b200moe_gemm_args* a, bool fc1);
 int nvfp4_small_gemm1(const b200moe_gemm_args* a, cudaStream_t stream);
 int nvfp4_small_gemm2(const b200moe_gemm_args* a, cudaStream_t stream);
 bool mx_small_batch_ok(const b200moe_gemm_args* a);
-bool mx_small_shape_ok(const b200moe_gemm_args* a);
+bool mx_small_tail_ok(const b200moe_gemm_args* a);
 int mx_small_gemm1(const b200moe_gemm_args* a, cudaStream_t stream, int tile_mode);
 int mx_small_gemm2(const b200moe_gemm_args* a, cudaStream_t stream, int tile_mode);
 bool pair_ok(const b200moe_gemm_args* a, bool fc1);
@@ -152,7 +152,7 @@ extern "C" int b200moe_grouped_gemm1_act(const b200moe_gemm_args* a, void* strea
       if (b200moe::pair_ok(a, /*fc1=*/true)) {
         const int rc1 = b200moe::mx_pair_gemm1(a, s);
         if (rc1 != B200MOE_OK || !b200moe::tail_split(a)) return rc1;
-        if (!b200moe::mx_small_shape_ok(a)) return b200moe::mx_gemm1(a, s, 1);
+        if (!b200moe::mx_small_tail_ok(a)) return b200moe::mx_gemm1(a, s, 1);
         const int rc2 = b200moe::mx_gemm1(a, s, 3);              // left-over tiles of more than 80 rows,
         return rc2 != B200MOE_OK ? rc2 : b200moe::mx_small_gemm1(a, s, 1);   // and the others
       }
@@ -183,7 +183,7 @@ extern "C" int b200moe_grouped_gemm2(const b200moe_gemm_args* a, void* stream) {
       if (b200moe::pair_ok(a, /*fc1=*/false)) {
         const int rc1 = b200moe::mx_pair_gemm2(a, s);
         if (rc1 != B200MOE_OK || !b200moe::tail_split(a)) return rc1;
-        if (!b200moe::mx_small_shape_ok(a)) return b200moe::mx_gemm2(a, s, 1);
+        if (!b200moe::mx_small_tail_ok(a)) return b200moe::mx_gemm2(a, s, 1);
         const int rc2 = b200moe::mx_gemm2(a, s, 3);              // left-over tiles of more than 80 rows,
         return rc2 != B200MOE_OK ? rc2 : b200moe::mx_small_gemm2(a, s, 1);   // and the others
       }

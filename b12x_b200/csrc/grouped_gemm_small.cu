@@ -662,22 +662,28 @@ bool nvfp4_small_batch_ok(const b200moe_gemm_args* a, bool fc1) {
   return true;
 }
 
-// w4a8_mx with a gated activation: plans that average up to 68 rows per expert, where nearly every expert
+// w4a8_mx with a gated activation: calls that average up to 68 rows per expert (the call's rows, not the plan's
+// capacity: all MX plans have the same 128-row tiles), where nearly every expert
 // is one tile of at most 80 columns; beyond, tiles of 64 read the weights twice and the 128-row kernel is
 // faster.  FC1 + FC2 of the GPT-OSS shape, 128-row kernel against this one: 32 tokens 243 : 203 us, 1024
 // (32 rows per expert) 390 : 319, 2048 (64) 412 : 360, 2200 (69) 413 : 364, 2400 (75) 415 : 418, 2600 (81)
 // 416 : 471.  Both wait for loads (some 2500 clocks from issue to landing); this kernel has five stages of
 // 16 KiB of weights in flight against four, since its token rows take 10 KiB of a stage instead of 16.
 // The left-over row tiles of the CTA-pair plans go here up to 80 rows (16384 tokens, FC1 + FC2 of the
-// tails 219 -> 179 us).  B200MOE_SMALL_BATCH=1 / 0 forces these kernels on / off.
-bool mx_small_shape_ok(const b200moe_gemm_args* a) {
+// tails 219 -> 179 us) where the call averages 256 rows per expert, as such plans do; below that the two
+// launches for left-over tiles would mostly find no work.  B200MOE_SMALL_BATCH=1 / 0 forces these kernels on / off.
+static int64_t call_rows(const b200moe_gemm_args* a) { return static_cast<int64_t>(a->num_tokens) * a->num_topk; }
+static bool mx_small_shape_ok(const b200moe_gemm_args* a) {
   if (small_batch_mode() == 0 || a->layout->tile_rows != 128 || a->activation == B200MOE_ACT_RELU2) return false;
   return a->hidden_size % 64 == 0 && a->intermediate % 64 == 0 && a->num_experts <= kMaxExperts;
 }
 bool mx_small_batch_ok(const b200moe_gemm_args* a) {
   const int mode = small_batch_mode();
   if (!mx_small_shape_ok(a)) return false;
-  return mode == 1 || static_cast<int64_t>(a->layout->rows) <= 68ll * a->num_experts;
+  return mode == 1 || call_rows(a) <= 68ll * a->num_experts;
+}
+bool mx_small_tail_ok(const b200moe_gemm_args* a) {
+  return mx_small_shape_ok(a) && call_rows(a) >= 256ll * a->num_experts;
 }
 
 int nvfp4_small_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {

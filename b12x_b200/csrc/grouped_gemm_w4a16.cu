@@ -1005,15 +1005,19 @@ static int launch(const TokenMaps& tmX, const CUtensorMap& tmW, const Params& p,
 // pairs beyond.  FC1 + FC2 of the Qwen3 shape, one CTA : narrow : wide, in us: 1 row per expert 185 : 200 :
 // 249, 16 rows 283 : 290 : 366, 24 rows 360 : 296 : 368, 48 rows 397 : 323 : 387, 56 rows 447 : 361 : 401,
 // 64 rows 564 : 444 : 421, 88 rows 759 : 583 : 454.
-// B200MOE_W4A16_PAIR=1 / 0 forces wide pairs / one CTA (2: narrow pairs).
-static int form_for(const b200moe_gemm_args* a) {
+// The rows are the call's, not the plan's capacity: the forms share one scratch layout, and a decode step
+// through a workspace planned for a prompt batch (layer, 16 tokens of 4096) took 273 us on wide pairs, 211
+// on one CTA.  B200MOE_W4A16_PAIR=1 / 0 forces wide pairs / one CTA (2: narrow pairs); a grid limited to one
+// CTA has no pair.
+static int form_for(const b200moe_gemm_args* a, int ctas) {
   static int mode = -2;
   if (mode == -2) {
     const char* e = getenv("B200MOE_W4A16_PAIR");
     mode = e == nullptr ? -1 : atoi(e);
   }
+  if (ctas < 2) return ONE;
   if (mode >= 0) return mode == 0 ? ONE : (mode == 2 ? PAIR_NARROW : PAIR_WIDE);
-  const int64_t rows = a->layout->rows, experts = a->num_experts;
+  const int64_t rows = static_cast<int64_t>(a->num_tokens) * a->num_topk, experts = a->num_experts;
   return rows < 18 * experts ? ONE : (rows < 58 * experts ? PAIR_NARROW : PAIR_WIDE);
 }
 
@@ -1031,7 +1035,7 @@ static int launch_any(const b200moe_gemm_args* a, const void* tokens, const void
   const int rc = make_tmap_bytes_2d(&tmW, weights, cols / 2, static_cast<uint64_t>(a->num_experts) * p.w_rows, 64);
   if (rc != B200MOE_OK) return rc;
   const int ctas = a->num_sms > 0 ? a->num_sms : num_sms_cached();
-  const int form = form_for(a);
+  const int form = form_for(a, ctas);
   p.n_tiles = form == ONE ? p.n_row_tiles : ceil_div_i(p.n_row_tiles, 2);
   if (form == ONE) return launch<EPI, ONE, kTo>(tmX, tmW, p, ctas, s);
   if (form == PAIR_NARROW) return launch<EPI, PAIR_NARROW, kTo>(tmX, tmW, p, ctas, s);

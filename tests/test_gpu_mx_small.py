@@ -31,3 +31,13 @@ def test_token_tiles(tokens, hidden, inter, act):
 @pytest.mark.parametrize("tokens", [257, 300, 335, 336, 337, 384, 600, 640])
 def test_left_over_row_tiles(tokens):
     _run(tokens, 1, 256, 192, "swigluoai")
+
+
+@pytest.mark.parametrize("tokens,planned", [(24, 1200), (300, 1200), (560, 1200)])   # 12, 150 and 280 rows per expert
+def test_small_calls_through_a_large_plan(tokens, planned):
+    """The call's rows choose the kernel; the plan's capacity does not change a bit of the result."""
+    shp = _mx(tokens=tokens, experts=2, topk=1, hidden=320, intermediate=192, activation="swigluoai")
+    inp = synth.make_inputs(shp, seed=tokens)
+    run = run_layer(inp, max_tokens=planned)
+    _check_mx_layer(run)
+    assert torch.equal(run.out_f32, run_layer(inp).out_f32)

@@ -3,7 +3,11 @@ steps on a CTA pair, at most 64 or 160), of their stages (two and four k-blocks 
 per-row power-of-two scaling of the FP16 token rows over the range of BF16."""
 
 import ctypes as C
+import os
+import subprocess
+import sys
 from dataclasses import replace
+from pathlib import Path
 
 import pytest
 import torch
@@ -151,3 +155,25 @@ def test_intermediate_rows_wider_than_fp16(tokens, experts):
     mid = taps.mid.abs()
     assert (mid.amax(dim=1) / mid.amin(dim=1)).min() > 2.0 ** 34
     _rowwise(run.out_f32, taps.out_f32, 1e-2)           # BF16 roundings of the intermediate that fall the other way
+
+
+@pytest.mark.parametrize("tokens,planned", [(20, 1200), (60, 1200), (200, 1200)])    # 10, 30 and 100 rows per expert
+def test_small_calls_through_a_large_plan(tokens, planned):
+    """The call's rows choose the form; the plan's capacity does not change a bit of the result."""
+    inp = synth.make_inputs(_w16(tokens=tokens, experts=2, topk=1, hidden=320, intermediate=192), seed=tokens)
+    run = run_layer(inp, max_tokens=planned)
+    _check_w4a16_layer(run)
+    assert torch.equal(run.out_f32, run_layer(inp).out_f32)
+
+
+@pytest.mark.timeout(300)
+def test_grid_of_one_cta():
+    """A persistent grid limited to one CTA cannot hold a pair: batches of every size run on the one-CTA form."""
+    if os.environ.get("B200MOE_NUM_SMS"):
+        pytest.skip("already the child run")
+    here = Path(__file__).resolve()
+    r = subprocess.run([sys.executable, "-m", "pytest", str(here), "-m", "gpu", "-q", "-p", "no:cacheprovider",
+                        "-k", "narrow_pair_token_tiles or cta_pair_token_tiles"],
+                       env=dict(os.environ, B200MOE_NUM_SMS="1"), capture_output=True, text=True, timeout=280,
+                       cwd=str(here.parent.parent))
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
