@@ -228,10 +228,10 @@ class MoERegime(str, Enum):
     materialized -- describe its SM120 kernels; every regime here materialises the routes with a
     separate sort and walks them with a persistent grid)."""
 
-    SMALL_BATCH = "small_batch_swap_ab"      # 64-row expert tiles, weights as the MMA rows (decode)
+    SMALL_BATCH = "small_batch_swap_ab"      # weights as the MMA rows, up to 64 / 80 token columns (decode)
     WIDE_TILE = "wide_tile"                  # 128 x 256 tiles, one CTA per tile
     WIDE_TILE_CTA_PAIR = "wide_tile_cta_pair"  # 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2)
-    W4A16_CONVERTER = "w4a16_converter"      # bf16 activations, FP4 weights expanded in shared memory
+    W4A16_CONVERTER = "w4a16_converter"      # bf16 activations, FP4 weights expanded into tensor memory (one CTA or pairs)
 
 
 class RouteLayout(str, Enum):
@@ -253,7 +253,7 @@ class GraphPartition(str, Enum):
 class GemmEngine(str, Enum):
     TCGEN05_MXF4NVF4 = "tcgen05_mxf4nvf4"    # nvfp4: E2M1 x E2M1, UE4M3 scale per 16
     TCGEN05_MXF8F6F4 = "tcgen05_mxf8f6f4"    # w4a8_mx: E4M3 x E2M1, UE8M0 scale per 32
-    TCGEN05_F16 = "tcgen05_f16"              # w4a16: bf16 x bf16 after in-kernel FP4 expansion
+    TCGEN05_F16 = "tcgen05_f16"              # w4a16: 16-bit operands after in-kernel FP4 expansion
 
 
 class PreparedWeightLayout(str, Enum):
@@ -308,31 +308,32 @@ class MoEExecutionPlan:
 
 def lower_moe_execution(spec: MoESpec, *, routed_rows_capacity: int, num_experts: int, intermediate_size: int,
                         hidden_size: int, tile_rows: int | None = None) -> MoEExecutionPlan:
-    """Regime and tile choice for one recipe and capacity -- the host-side statement of what the
-    C ABI decides (``b200moe_scratch_nbytes`` for the tile height, the GEMM entry points for the
-    kernel family).  ``tile_rows`` overrides the tile height (64 / 128)."""
+    """Regime and tile choice for one recipe and number of routed rows -- the host-side statement of what the
+    C ABI decides for a call of that many rows (``b200moe_scratch_nbytes`` for the tile height, the GEMM entry
+    points for the kernel family; w4a16 and the w4a8_mx small-batch kernel go by the rows of the call, so a
+    smaller call through the same plan may run another one).  ``tile_rows`` overrides the tile height (64 / 128)."""
     rows, e = int(routed_rows_capacity), int(num_experts)
     gated = spec.activation in GATED_ACTIVATIONS
     small_ok = spec.quant_mode == "nvfp4" and intermediate_size % 128 == 0 and hidden_size % 64 == 0
     tm = int(tile_rows) if tile_rows else (64 if (small_ok and rows <= 48 * e) else 128)
     if tm == 64 and not small_ok:
         tm = 128
+    pair_ok = gated and intermediate_size % 64 == 0 and hidden_size % 64 == 0
+    regime, tile_m, tile_n = MoERegime.WIDE_TILE, tm, 256
     if spec.quant_mode == "w4a16":
         regime, engine = MoERegime.W4A16_CONVERTER, GemmEngine.TCGEN05_F16
-    elif spec.quant_mode == "w4a8_mx":
-        regime, engine = MoERegime.WIDE_TILE, GemmEngine.TCGEN05_MXF8F6F4
+        tile_m = 64 if rows < 58 * e else 160           # token columns; weight rows: one CTA, or a pair
+        tile_n = 128 if rows < 18 * e else 256
     else:
-        engine = GemmEngine.TCGEN05_MXF4NVF4
-        if tm == 64:
-            regime = MoERegime.SMALL_BATCH
-        elif gated and rows >= 256 * e:
-            regime = MoERegime.WIDE_TILE_CTA_PAIR
-        else:
-            regime = MoERegime.WIDE_TILE
+        mx = spec.quant_mode == "w4a8_mx"
+        engine = GemmEngine.TCGEN05_MXF8F6F4 if mx else GemmEngine.TCGEN05_MXF4NVF4
+        if tm == 64 or (mx and pair_ok and rows <= 68 * e):
+            regime, tile_m = MoERegime.SMALL_BATCH, 80 if mx else 64
+        elif pair_ok and rows >= 256 * e:
+            regime, tile_m = MoERegime.WIDE_TILE_CTA_PAIR, 256
     return MoEExecutionPlan(
         regime=regime, route_layout=RouteLayout.SORTED_COMPACT_EXPERT,
         work_availability=WorkAvailability.PRECOMPUTED, scheduler=WorkScheduler.PERSISTENT_GRID,
         graph_partition=GraphPartition.SPLIT_FC1_FC2, gemm_engine=engine,
         weight_layout=PreparedWeightLayout.SOURCE_NATIVE, reduction=OutputReduction.ROUTE_BUFFER_TOPK_SUM,
-        tile_m=256 if regime is MoERegime.WIDE_TILE_CTA_PAIR else tm,
-        tile_n=256, route_block_rows=tm)
+        tile_m=tile_m, tile_n=tile_n, route_block_rows=tm)

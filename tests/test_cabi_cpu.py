@@ -145,6 +145,22 @@ def test_caps_plan_and_required_nbytes_agree(lib):
     assert (oai.swiglu_limit, oai.swiglu_alpha, oai.swiglu_beta) == (7.0, 1.702, 1.0)
 
 
+@pytest.mark.parametrize("mode,source,tokens,regime,tile", [
+    ("w4a8_mx", "fp4_e8m0_k32", 136, "small_batch_swap_ab", (80, 256)),       # 68 rows per expert
+    ("w4a8_mx", "fp4_e8m0_k32", 137, "wide_tile", (128, 256)),
+    ("w4a8_mx", "fp4_e8m0_k32", 512, "wide_tile_cta_pair", (256, 256)),       # 256
+    ("nvfp4", "modelopt_nvfp4", 96, "small_batch_swap_ab", (64, 256)),        # 48
+    ("nvfp4", "modelopt_nvfp4", 97, "wide_tile", (128, 256)),
+    ("w4a16", "modelopt_nvfp4", 35, "w4a16_converter", (64, 128)),            # below 18
+    ("w4a16", "modelopt_nvfp4", 36, "w4a16_converter", (64, 256)),
+    ("w4a16", "modelopt_nvfp4", 116, "w4a16_converter", (160, 256)),          # 58
+])
+def test_plan_execution_names_the_kernel_that_runs(mode, source, tokens, regime, tile):
+    wp = _wplan(quant_modes=mode, source_format=source)
+    p = fused_moe.plan_execution(num_tokens=tokens, num_topk=wp.num_experts // 2, device="cpu", weight_plan=wp, quant_mode=mode)
+    assert (p.execution.regime.value, (p.tile_m, p.tile_n)) == (regime, tile)
+
+
 def _cpu_experts(wp):
     e, k, i = wp.num_experts, wp.hidden_size, wp.intermediate_size
     return fused_moe.prepare_weights(
