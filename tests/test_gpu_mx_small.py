@@ -6,8 +6,10 @@ import pytest
 import torch
 
 from b12x_b200 import synth
+from oracle import moe_oracle as O
 from tests.gpu_utils import run_layer
-from tests.test_gpu_parity import _check_mx_layer, _mx
+from tests.helpers import atoms_to_rows
+from tests.test_gpu_parity import FLIP_TOL, _check_mx_layer, _mx
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +43,24 @@ def test_small_calls_through_a_large_plan(tokens, planned):
     run = run_layer(inp, max_tokens=planned)
     _check_mx_layer(run)
     assert torch.equal(run.out_f32, run_layer(inp).out_f32)
+
+
+@pytest.mark.parametrize("tokens", [17, 80, 150])
+@pytest.mark.parametrize("limit,act", [(0.5, "silu"), (None, "situ")])
+def test_other_gated_epilogues(tokens, limit, act):
+    """SwiGLU with a clamp that cuts many values, and SiTU: FC1's stored MXFP8 rows against the tap's activation."""
+    shp = _mx(tokens=tokens, experts=4, topk=1, hidden=320, intermediate=192, activation=act)
+    inp = synth.make_inputs(shp, seed=tokens)
+    run = run_layer(inp, topk_ids=torch.full((tokens, 1), 2, dtype=torch.int32), topk_weights=torch.ones(tokens, 1),
+                    swiglu_limit=limit)
+    b = run.binding
+    f = run.fc1[:tokens]
+    if limit is not None:
+        assert float((f.abs() > limit).float().mean()) > 0.05
+    codes, scales, _ = O.quantize_mxfp8_rows(O.gated_activation(f[:, 192:], f[:, :192], act, limit, 1.0, 0.0))
+    # the kernel's exponential and reciprocal are an ulp or two off torch's: codes at a rounding boundary may flip
+    assert float((b.materialized_intermediate.cpu()[:tokens] != codes).float().mean()) <= FLIP_TOL
+    sf = b.intermediate_scale.cpu()
+    for mt in range((tokens + 127) // 128):
+        rows = slice(128 * mt, min(tokens, 128 * mt + 128))
+        assert torch.equal(atoms_to_rows(sf, mt, 2, rows.stop - rows.start, 6), scales[rows])

@@ -1,9 +1,7 @@
-"""-m gpu: W4A16 layers with several 128-row tiles per expert against the CPU oracle.  In-process the
-kernel family follows the plan (CTA pairs once it averages two row tiles per expert); the two child
-runs repeat this file and the other W4A16 cases with the CTA-pair kernels forced on
-(B200MOE_W4A16_PAIR=1: every shape, also experts with one or an odd number of row tiles -- once with
-the left-over row tile on a single-CTA launch, B200MOE_TAIL_SPLIT=1, once as half of a pair, =0) and
-off (=0: the single-CTA kernel).  The switch is read once per process."""
+"""-m gpu: W4A16 layers with several token tiles per expert against the CPU oracle.  In-process the form
+follows the rows per expert (one CTA, narrow or wide CTA pairs); the child runs repeat this file and the
+other W4A16 cases (gated and relu2, several unequal experts, E8M0 scales) with every shape on one form:
+B200MOE_W4A16_PAIR=0 one CTA, =1 wide pairs, =2 narrow pairs.  The switch is read once per process."""
 
 import os
 import subprocess
@@ -20,9 +18,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("tokens,experts,topk,hidden,inter,act", [
-    (700, 4, 2, 512, 256, "silu"),          # 2-3 row tiles per expert, 4 feature tiles, one code box
-    (300, 2, 2, 640, 384, "silu"),          # 6 k-blocks in FC2: a full and a half box of codes
-    (260, 1, 1, 320, 192, "silu"),          # 320 output features: the last feature tile is half empty
+    (700, 4, 2, 512, 256, "silu"),          # 2-3 wide token tiles per expert, one code stage in FC2
+    (300, 2, 2, 640, 384, "silu"),          # 6 k-blocks in FC2: a full and a half stage of codes
+    (260, 1, 1, 320, 192, "silu"),          # 320 output features: the last weight tile is half empty
     (150, 2, 1, 256, 448, "relu2"),         # 7 k-blocks
 ])
 def test_w4a16_multi_tile_matches_oracle(tokens, experts, topk, hidden, inter, act):
@@ -31,21 +29,21 @@ def test_w4a16_multi_tile_matches_oracle(tokens, experts, topk, hidden, inter, a
 
 
 @pytest.mark.parametrize("tokens,experts,topk,hidden,inter,act", [
-    (1100, 4, 2, 512, 256, "silu"),         # 4-5 row tiles per expert: full pairs and a half-empty one
-    (640, 1, 1, 256, 192, "silu"),          # exactly five row tiles, one and a half feature tiles
+    (1100, 4, 2, 512, 256, "silu"),         # 3-4 wide token tiles per expert, 8-9 narrow ones
+    (640, 1, 1, 256, 192, "silu"),          # exactly four wide token tiles, ten narrow ones
 ])
 def test_w4a16_many_row_tiles_matches_oracle(tokens, experts, topk, hidden, inter, act):
     shp = _w16(tokens=tokens, experts=experts, topk=topk, hidden=hidden, intermediate=inter, activation=act)
     _check_w4a16_layer(run_layer(synth.make_inputs(shp, seed=tokens + inter), want_fc1=True))
 
 
-@pytest.mark.parametrize("pair,split", [("1", "1"), ("1", "0"), ("0", "1")])
+@pytest.mark.parametrize("form", ["0", "1", "2"])
 @pytest.mark.timeout(900)
-def test_both_kernel_families_pass_the_w4a16_cases(pair, split):
+def test_every_form_passes_the_w4a16_cases(form):
     if os.environ.get("B200MOE_W4A16_CHILD") == "1":
         pytest.skip("already the child run")
     here = Path(__file__).resolve().parent
-    env = dict(os.environ, B200MOE_W4A16_PAIR=pair, B200MOE_TAIL_SPLIT=split, B200MOE_W4A16_CHILD="1")
+    env = dict(os.environ, B200MOE_W4A16_PAIR=form, B200MOE_W4A16_CHILD="1")
     r = subprocess.run([sys.executable, "-m", "pytest", str(Path(__file__).resolve()),
                         str(here / "test_gpu_parity.py"), str(here / "test_w4a16_sources.py"),
                         "-m", "gpu", "-k", "w4a16", "-x", "-q", "-p", "no:cacheprovider"],
