@@ -644,8 +644,8 @@ static int token_maps(CUtensorMap (&tmX)[3], const void* base, uint64_t row_byte
 
 }  // namespace small
 
-// The small-batch kernels serve plans cut into 64-row tiles.  B200MOE_SMALL_BATCH=0 keeps the
-// wide-tile kernels on such plans (comparison runs).
+// The small-batch kernels serve nvfp4 plans cut into 64-row tiles and small w4a8_mx calls (see below).
+// B200MOE_SMALL_BATCH=0 keeps the wide-tile kernels on both (comparison runs).
 static int small_batch_mode() {
   static int mode = -2;
   if (mode == -2) {

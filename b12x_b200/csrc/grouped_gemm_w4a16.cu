@@ -1,5 +1,5 @@
 // Grouped expert GEMMs of the w4a16 recipe: BF16 activations x NVFP4 (or MXFP4) weights that are
-// expanded to BF16 on the fly, on tcgen05.mma.kind::f16 with FP32 accumulation in TMEM.
+// expanded to 16 bits on the fly, on tcgen05.mma.kind::f16 with FP32 accumulation in TMEM.
 //
 // The tensor core cannot read 4-bit operands next to 16-bit ones, so the main loop has a conversion
 // step, and how often a weight is converted, and how much of a tile is padding, decides the time.
@@ -7,7 +7,7 @@
 // columns, any multiple of 16:
 //   * an expert with 2 rows costs 16 columns and one with 270 costs 2 x 144: with the tokens as the
 //     128 rows of a tile (what this kernel replaces) the first cost 128 and the second 384;
-//   * a converter thread owns one weight row = one TMEM lane and stores its BF16 values straight
+//   * a converter thread owns one weight row = one TMEM lane and stores its 16-bit values straight
 //     into tensor memory (tcgen05.st), where the MMA takes its A operand from: no shared-memory
 //     round trip, no proxy fence.
 // FC1 with a gated activation interleaves the operand rows: lanes 0..15 of every warp hold 16 up
@@ -120,7 +120,8 @@ template <int kForm>
 constexpr int smem_bytes() {
   return 1024 + Cfg<kForm>::kRawStages * kSmemRaw + Cfg<kForm>::kSmemTok + static_cast<int>(sizeof(SmemTail));
 }
-static_assert(smem_bytes<ONE>() <= 227 * 1024 && smem_bytes<PAIR_WIDE>() <= 227 * 1024, "shared memory of the W4A16 kernel");
+static_assert(smem_bytes<ONE>() <= 227 * 1024 && smem_bytes<PAIR_NARROW>() <= 227 * 1024 &&
+                  smem_bytes<PAIR_WIDE>() <= 227 * 1024, "shared memory of the W4A16 kernel");
 
 enum { EPI_FC1_GATED = 0, EPI_FC1_RELU2 = 1, EPI_FC2 = 2 };
 
@@ -134,7 +135,7 @@ struct Params {
   float* tap;
   const float* route_weights;    // FC1, optional: per flat route, multiplies the route's row with its alpha
   const int32_t* sorted_route_ids;
-  int E, n_tiles, kdim, k_blocks, atoms_k, sf_rowgroups, w_rows;
+  int E, n_tiles, k_blocks, atoms_k, sf_rowgroups, w_rows;
   int sub0_base, sub1_base;      // first weight row of the two 64-row sub-tiles at weight tile 0
   int n_step;                    // weight rows a sub-tile advances per weight tile
   int out_cols;
@@ -556,8 +557,6 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
     const int row = kGated ? 16 * sub + (lane & 15) + 64 * (lane >> 4) : 32 * sub + lane;
     const uint32_t a_lane = tmem_base + C::kRingCol + (static_cast<uint32_t>(sub * 32) << 16);
     const uint32_t afull0 = kPair ? map_to_cta(smem_u32(&tail->afull[0]), 0) : 0u;
-    int rs = 0;
-    uint32_t rphase = 0;
     const uint32_t chunk_xor = static_cast<uint32_t>(row & 7) << 4;
     const int n_raw = (p.k_blocks + kKBlocksPerRaw - 1) / kKBlocksPerRaw, n_stages = (p.k_blocks + C::kStageKb - 1) / C::kStageKb;
     uint32_t raw0 = 0, stage0 = 0;   // raw stages and MMA stages before this tile
@@ -574,89 +573,89 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       const uint32_t sf_off = kSmemCodes + min(slot, 3) * 2048 + (wrow & 31) * 16 + ((wrow >> 5) & 3) * 4;
       // the two groups take the raw stages in turn
       auto convert = [&](auto as_bf16) {
-      constexpr bool kBf16 = decltype(as_bf16)::value;     // TO_F16: re-encode for an expert marked `wide`
-      for (int r = (group + raw0) & 1; r < n_raw; r += kConvGroups) {
-        const uint32_t rs = (raw0 + r) % C::kRawStages, rphase = ((raw0 + r) / C::kRawStages) & 1u;
-        if (!mbar_wait_bounded(&tail->rfull[rs], rphase, abort_flag, p.status, WAIT_CONVERT)) {
-          ok = false;
-          break;
-        }
-        const uint8_t* raw = sRaw + rs * kSmemRaw;
-        const uint8_t* codes = raw + row * 128;
-        const int nk = min(kKBlocksPerRaw, p.k_blocks - r * kKBlocksPerRaw);
-#pragma unroll
-        for (int q = 0; q < kKBlocksPerRaw / C::kStageKb; ++q) {   // the one or two MMA stages of the raw stage
-          if (C::kStageKb * q >= nk) break;
-          const uint32_t si = stage0 + (kKBlocksPerRaw / C::kStageKb) * r + q;
-          const uint32_t as = si % C::kRing, aphase = (si / C::kRing) & 1u;
-          if (!mbar_wait_bounded(&tail->aempty[as], aphase ^ 1, abort_flag, p.status, WAIT_CONVERT)) {
+        constexpr bool kBf16 = decltype(as_bf16)::value;     // TO_F16: re-encode for an expert marked `wide`
+        for (int r = (group + raw0) & 1; r < n_raw; r += kConvGroups) {
+          const uint32_t rs = (raw0 + r) % C::kRawStages, rphase = ((raw0 + r) / C::kRawStages) & 1u;
+          if (!mbar_wait_bounded(&tail->rfull[rs], rphase, abort_flag, p.status, WAIT_CONVERT)) {
             ok = false;
             break;
           }
-          tc_fence_after();
-          const uint32_t a_t = a_lane + as * C::kStageCols;
-          // the k-blocks of the stage (missing ones: unread values); the next one's codes are fetched
-          // ahead of this one's stores
-          const int k0 = C::kStageKb * q;
-          uint4 nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * k0 << 4) ^ chunk_xor));
-          uint4 nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * k0 + 1) << 4) ^ chunk_xor));
-          uint32_t nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + k0 * 512);
+          const uint8_t* raw = sRaw + rs * kSmemRaw;
+          const uint8_t* codes = raw + row * 128;
+          const int nk = min(kKBlocksPerRaw, p.k_blocks - r * kKBlocksPerRaw);
 #pragma unroll
-          for (int hk = 0; hk < C::kStageKb; ++hk) {
-            const uint4 cw[2] = {nx0, nx1};
-            const uint32_t sfw = nsf;
-            if (hk + 1 < C::kStageKb) {
-              nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * (k0 + hk + 1) << 4) ^ chunk_xor));
-              nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * (k0 + hk + 1) + 1) << 4) ^ chunk_xor));
-              nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + (k0 + hk + 1) * 512);
+          for (int q = 0; q < kKBlocksPerRaw / C::kStageKb; ++q) {   // the one or two MMA stages of the raw stage
+            if (C::kStageKb * q >= nk) break;
+            const uint32_t si = stage0 + (kKBlocksPerRaw / C::kStageKb) * r + q;
+            const uint32_t as = si % C::kRing, aphase = (si / C::kRing) & 1u;
+            if (!mbar_wait_bounded(&tail->aempty[as], aphase ^ 1, abort_flag, p.status, WAIT_CONVERT)) {
+              ok = false;
+              break;
             }
-            uint32_t s01 = 0, s23 = 0;
-            if (kTo == TO_F16) cvt_e4m3x4_f16(sfw, s01, s23);
+            tc_fence_after();
+            const uint32_t a_t = a_lane + as * C::kStageCols;
+            // the k-blocks of the stage (missing ones: unread values); the next one's codes are fetched
+            // ahead of this one's stores
+            const int k0 = C::kStageKb * q;
+            uint4 nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * k0 << 4) ^ chunk_xor));
+            uint4 nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * k0 + 1) << 4) ^ chunk_xor));
+            uint32_t nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + k0 * 512);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {                    // 32 codes -> 16 TMEM columns
-              const uint4 v = cw[h];
-              const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-              uint32_t out[16];
-#pragma unroll
-              for (int b = 0; b < 2; ++b) {                  // 16 values per scale
-                uint32_t o0[4], o1[4];
-                if (kTo == TO_F16) {
-                  const uint32_t sc = __byte_perm(h == 0 ? s01 : s23, 0u, b == 0 ? 0x1010u : 0x3232u);
-                  cvt_e2m1x8_scaled_f16(words[2 * b], sc, o0);
-                  cvt_e2m1x8_scaled_f16(words[2 * b + 1], sc, o1);
-                } else {
-                  const uint32_t sb = (sfw >> (16 * h + 8 * b)) & 0xffu;
-                  // E8M0: 2^(b-127) is the f32 with exponent field b (b = 0: the subnormal 2^-127)
-                  const __nv_bfloat16 s1 = __float2bfloat16_rn(__uint_as_float(sb != 0u ? sb << 23 : 0x00400000u));
-                  const __nv_bfloat162 sc = __halves2bfloat162(s1, s1);
-                  cvt_e2m1x8_bf16(words[2 * b], sc, o0);
-                  cvt_e2m1x8_bf16(words[2 * b + 1], sc, o1);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  out[8 * b + i] = o0[i];
-                  out[8 * b + 4 + i] = o1[i];
-                }
+            for (int hk = 0; hk < C::kStageKb; ++hk) {
+              const uint4 cw[2] = {nx0, nx1};
+              const uint32_t sfw = nsf;
+              if (hk + 1 < C::kStageKb) {
+                nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * (k0 + hk + 1) << 4) ^ chunk_xor));
+                nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * (k0 + hk + 1) + 1) << 4) ^ chunk_xor));
+                nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + (k0 + hk + 1) * 512);
               }
-              if (kBf16) {
+              uint32_t s01 = 0, s23 = 0;
+              if (kTo == TO_F16) cvt_e4m3x4_f16(sfw, s01, s23);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) out[i] = f16x2_to_bf16x2(out[i]);
+              for (int h = 0; h < 2; ++h) {                    // 32 codes -> 16 TMEM columns
+                const uint4 v = cw[h];
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+                uint32_t out[16];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {                  // 16 values per scale
+                  uint32_t o0[4], o1[4];
+                  if (kTo == TO_F16) {
+                    const uint32_t sc = __byte_perm(h == 0 ? s01 : s23, 0u, b == 0 ? 0x1010u : 0x3232u);
+                    cvt_e2m1x8_scaled_f16(words[2 * b], sc, o0);
+                    cvt_e2m1x8_scaled_f16(words[2 * b + 1], sc, o1);
+                  } else {
+                    const uint32_t sb = (sfw >> (16 * h + 8 * b)) & 0xffu;
+                    // E8M0: 2^(b-127) is the f32 with exponent field b (b = 0: the subnormal 2^-127)
+                    const __nv_bfloat16 s1 = __float2bfloat16_rn(__uint_as_float(sb != 0u ? sb << 23 : 0x00400000u));
+                    const __nv_bfloat162 sc = __halves2bfloat162(s1, s1);
+                    cvt_e2m1x8_bf16(words[2 * b], sc, o0);
+                    cvt_e2m1x8_bf16(words[2 * b + 1], sc, o1);
+                  }
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    out[8 * b + i] = o0[i];
+                    out[8 * b + 4 + i] = o1[i];
+                  }
+                }
+                if (kBf16) {
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) out[i] = f16x2_to_bf16x2(out[i]);
+                }
+                tc_st_32x32b_x16(a_t + 32 * hk + 16 * h, out);
               }
-              tc_st_32x32b_x16(a_t + 32 * hk + 16 * h, out);
+            }
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if (kPair) mbar_arrive_cluster(afull0 + as * static_cast<uint32_t>(sizeof(uint64_t)));
+              else mbar_arrive(&tail->afull[as]);
             }
           }
-          tc_wait_st();
-          tc_fence_before();
+          // this warp has read all it needs of the stage's codes and atoms
           __syncwarp();
-          if (lane == 0) {
-            if (kPair) mbar_arrive_cluster(afull0 + as * static_cast<uint32_t>(sizeof(uint64_t)));
-            else mbar_arrive(&tail->afull[as]);
-          }
+          if (lane == 0) mbar_arrive(&tail->rempty[rs]);
         }
-        // this warp has read all it needs of the stage's codes and atoms
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tail->rempty[rs]);
-      }
       };
       if (kTo == TO_F16 && c.wide) convert(std::true_type{});
       else convert(std::false_type{});
@@ -1103,7 +1102,6 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
   p.tap = a->fc1_tap;
   p.route_weights = a->fc1_route_weights;
   p.sorted_route_ids = reinterpret_cast<const int32_t*>(base + L.sorted_route_ids);
-  p.kdim = K;
   p.k_blocks = K / kKPerBlock;
   p.atoms_k = ceil_div_i(K, 64);
   p.sf_rowgroups = ceil_div_i(w_rows, 128);
@@ -1136,7 +1134,6 @@ int w4a16_gemm2(const b200moe_gemm_args* a, cudaStream_t stream) {
   p.sf = a->w2_sf;
   p.alphas = a->w2_alphas;
   p.out_f32 = reinterpret_cast<float*>(base + L.routed);
-  p.kdim = I;
   p.k_blocks = I / kKPerBlock;
   p.atoms_k = ceil_div_i(I, 64);
   p.sf_rowgroups = ceil_div_i(K, 128);
