@@ -667,7 +667,9 @@ bool nvfp4_small_batch_ok(const b200moe_gemm_args* a, bool fc1) {
 // is one tile of at most 80 columns; beyond, tiles of 64 read the weights twice and the 128-row kernel is
 // faster.  FC1 + FC2 of the GPT-OSS shape, 128-row kernel against this one: 32 tokens 243 : 203 us, 1024
 // (32 rows per expert) 390 : 319, 2048 (64) 412 : 360, 2200 (69) 413 : 364, 2400 (75) 415 : 418, 2600 (81)
-// 416 : 471.  Both wait for loads (some 2500 clocks from issue to landing); this kernel has five stages of
+// 416 : 471.  On other shapes up to the limit this kernel takes 0.65 to 0.99 of the 128-row kernel's time (layer; 256
+// experts of 7168 x 2048, 64 tokens 1264 : 852 us; 8 of 4096 x 14336, 256 tokens 200 : 171), 1.02 on a layer of 4 experts
+// of 256 x 128.  Both wait for loads (some 2500 clocks from issue to landing); this kernel has five stages of
 // 16 KiB of weights in flight against four, since its token rows take 10 KiB of a stage instead of 16.
 // The left-over row tiles of the CTA-pair plans go here up to 80 rows (16384 tokens, FC1 + FC2 of the
 // tails 219 -> 179 us) where the call averages 256 rows per expert, as such plans do; below that the two

@@ -1003,7 +1003,10 @@ static int launch(const TokenMaps& tmX, const CUtensorMap& tmW, const Params& p,
 // expert is one tile of at most 64 columns; one wait of the MMA thread covers 256 rows x 256 values), wide
 // pairs beyond.  FC1 + FC2 of the Qwen3 shape, one CTA : narrow : wide, in us: 1 row per expert 185 : 200 :
 // 249, 16 rows 283 : 290 : 366, 24 rows 360 : 296 : 368, 48 rows 397 : 323 : 387, 56 rows 447 : 361 : 401,
-// 64 rows 564 : 444 : 421, 88 rows 759 : 583 : 454.
+// 64 rows 564 : 444 : 421, 88 rows 759 : 583 : 454.  The lines lie in the same place elsewhere (layer, us): 128 experts
+// of 2880 x 2880, 18 / 24 / 58 / 64 rows 423 / 535 / 701 / 840 : 461 / 473 / 623 / 734 : 543 / 551 / 637 / 674; 256 of
+// 7168 x 256 282 / 351 / 576 / 636 : 288 / 318 / 531 / 584 : 317 / 343 / 520 / 538; 8 of 4096 x 3584 88 / 98 / 112 /
+// 132 : 96 / 98 / 102 / 115 : 102 / 105 / 111 / 118.
 // The rows are the call's, not the plan's capacity: the forms share one scratch layout, and a decode step
 // through a workspace planned for a prompt batch (layer, 16 tokens of 4096) took 273 us on wide pairs, 211
 // on one CTA.  B200MOE_W4A16_PAIR=1 / 0 forces wide pairs / one CTA (2: narrow pairs); a grid limited to one
