@@ -28,8 +28,9 @@
 // clock and SM against 70 to 77; so the MMA runs on FP16 x FP16 and the token rows come as FP16,
 // scaled by a power of two per row (permute_rows_f16_kernel), which BF16 values survive unchanged.
 // E8M0 scales exceed the FP16 range: with them both operands are BF16.  So they are for an expert one of
-// whose rows spans more binades than FP16 carries exactly (permute_rows_f16_kernel marks it): its items
-// take the BF16 rows and re-encode the weights, at the lower rate.
+// whose rows spans more binades than FP16 carries exactly (permute_rows_f16_kernel marks it): the kernel
+// takes the other experts first and then, if there are marks, the marked ones with the same roles on BF16 rows
+// and re-encoded weights, at the lower rate.  (Of 50 million values of a SwiGLU some ten lie that close to zero.)
 //
 // What bounds it and what it took, on the Qwen3-235B shape (K 4096, I 1536, 128 experts, top-8),
 // FC1 / FC2 in microseconds:
@@ -77,8 +78,8 @@ constexpr int kTmemCols = 512;
 constexpr int kMaxList = 256;               // work items a CTA decodes ahead of its main loop
 
 // What the weights are expanded to: FP16 (E4M3 scales; the token rows then are FP16 too, scaled by a
-// power of two per row), or BF16 (E8M0 scales, which exceed the FP16 range).
-enum { TO_F16 = 0, TO_BF16_E8M0 = 1 };
+// power of two per row), or BF16 (E8M0 scales, which exceed the FP16 range; E4M3 scales of marked experts).
+enum { TO_F16 = 0, TO_BF16_E8M0 = 1, TO_BF16_E4M3 = 2 };
 
 // A stage is what one wait and one commit of the MMA thread cover.
 // ONE: one CTA, 2 x 64 accumulator columns + 3 converted stages of four k-blocks (128 columns each).
@@ -100,7 +101,7 @@ struct Cfg {
   static_assert(kRingCol + kStageCols * kRing <= kTmemCols, "tensor memory");
 };
 
-struct __align__(16) SmemTail {
+struct Bars {
   uint64_t rfull[6];    // packed codes and scale atoms landed
   uint64_t rempty[6];   // ... read by the group that converts them
   uint64_t tfull[kTokStagesMax];             // token rows landed (pair: both halves, on the even CTA)
@@ -109,12 +110,17 @@ struct __align__(16) SmemTail {
   uint64_t aempty[4];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+};
+struct __align__(16) SmemTail {
+  Bars bars[2];                         // of the unmarked and of the marked experts' run
   uint32_t tmem_base;
   int abort_flag;
-  int max_cols;                         // of all tiles of the launch
-  int32_t tile_base[kMaxExperts + 1];   // token tiles before expert e
+  int max_cols;                         // of all tiles of the run
+  int any_wide;                         // some experts are marked
+  int32_t tile_base[kMaxExperts + 1];   // token tiles before expert e (of the run's experts)
+  uint8_t wide[kMaxExperts];
   int32_t offs[kMaxExperts + 1];        // first sorted row of expert e
-  int4 list[kMaxList];                  // this CTA's first work items: {expert (+ kWideBit), weight tile, row0, nrows}
+  int4 list[kMaxList];                  // this CTA's first work items: {expert, weight tile, row0, nrows}
 };
 template <int kForm>
 constexpr int smem_bytes() {
@@ -143,23 +149,15 @@ struct Params {
   float limit, act_alpha, act_beta;
   int swigluoai;
   const float* row_inv;          // TO_F16: per sorted row, the power of two that undoes its scaling
-  const int32_t* wide;           // TO_F16: per expert, nonzero = BF16 operands
-};
-
-// Token rows, one map per box height: 64, 32 and 16 rows.  [0] the rows as `kTo` says, [1] TO_F16: the
-// same rows as BF16, for experts marked `wide`.
-struct TokenMaps {
-  CUtensorMap m[2][3];
+  const int32_t* wide;           // TO_F16: per expert, nonzero = marked
 };
 
 // A work item: expert, weight tile, and the token rows [row0, row0 + nrows) of the expert.  An
 // expert's rows are cut evenly into as few tiles as the column limit allows.
 struct Work {
   int e, nt, row0, nrows, cols;
-  bool wide;
 };
-constexpr int kWideBit = 1 << 16;      // of a listed item's expert
-template <int kForm, int kTo>
+template <int kForm>
 __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTail* tail, int rank) {
   const int32_t* tb = tail->tile_base;
   const int q = w / p.n_tiles;
@@ -180,18 +178,16 @@ __device__ __forceinline__ Work decode_work(int w, const Params& p, const SmemTa
   c.row0 = first + mt * step;
   c.nrows = min(step, cnt - mt * step);
   c.cols = (c.nrows + kStep - 1) & ~(kStep - 1);
-  c.wide = kTo == TO_F16 && p.wide[lo] != 0;
   return c;
 }
 // the i-th item of this CTA, w = its number: out of the list the CTA made at its start where that reaches
-template <int kForm, int kTo>
+template <int kForm>
 __device__ __forceinline__ Work get_work(int i, int w, const Params& p, const SmemTail* tail, int rank) {
-  if (i >= kMaxList) return decode_work<kForm, kTo>(w, p, tail, rank);
+  if (i >= kMaxList) return decode_work<kForm>(w, p, tail, rank);
   const int4 v = tail->list[i];
   constexpr int kStep = Cfg<kForm>::kColStep;
   Work c;
-  c.e = v.x & (kWideBit - 1);
-  c.wide = kTo == TO_F16 && v.x >= kWideBit;
+  c.e = v.x;
   c.nt = v.y;
   c.row0 = v.z;
   c.nrows = v.w;
@@ -292,66 +288,54 @@ __device__ __forceinline__ void mma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tme
       : "memory");
 }
 
-template <int EPI, int kForm, int kTo>
-__global__ void __launch_bounds__(kThreads, 1)
-grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_constant__ CUtensorMap tmW,
-                          const Params p) {
+template <int kForm>
+__device__ __forceinline__ void init_bars(Bars* bars) {
   using C = Cfg<kForm>;
-  constexpr bool kPair = C::kPair;
-  constexpr bool kGated = EPI == EPI_FC1_GATED;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  uint8_t* sTok = smem;
-  uint8_t* sRaw = sTok + C::kSmemTok;
-  SmemTail* tail = reinterpret_cast<SmemTail*>(sRaw + C::kRawStages * kSmemRaw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = kPair ? static_cast<int>(cluster_ctarank()) : 0;
+  for (int s = 0; s < C::kRawStages; ++s) {
+    mbar_init(&bars->rfull[s], 1);
+    mbar_init(&bars->rempty[s], 4);      // the group that converts the stage
+  }
+  for (int s = 0; s < kTokStagesMax; ++s) {
+    mbar_init(&bars->tfull[s], 1);
+    mbar_init(&bars->tempty[s], 1);
+  }
+  for (int s = 0; s < C::kRing; ++s) {
+    mbar_init(&bars->afull[s], C::kPair ? 8 : 4);
+    mbar_init(&bars->aempty[s], 1);
+  }
+  for (int b = 0; b < 2; ++b) {
+    mbar_init(&bars->acc_full[b], 1);
+    mbar_init(&bars->acc_empty[b], C::kPair ? 2 * kEpiWarps : kEpiWarps);
+  }
+  fence_mbar_init();
+}
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < C::kRawStages; ++s) {
-      mbar_init(&tail->rfull[s], 1);
-      mbar_init(&tail->rempty[s], 4);      // the group that converts the stage
-    }
-    for (int s = 0; s < kTokStagesMax; ++s) {
-      mbar_init(&tail->tfull[s], 1);
-      mbar_init(&tail->tempty[s], 1);
-    }
-    for (int s = 0; s < C::kRing; ++s) {
-      mbar_init(&tail->afull[s], kPair ? 8 : 4);
-      mbar_init(&tail->aempty[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&tail->acc_full[b], 1);
-      mbar_init(&tail->acc_empty[b], kPair ? 2 * kEpiWarps : kEpiWarps);
-    }
-    tail->abort_flag = 0;
-    fence_mbar_init();
-  }
-  for (int i = threadIdx.x; i <= p.E; i += kThreads) tail->offs[i] = p.expert_offsets[i];
-  if (warp == 1) {
-    if (kPair) {
-      tmem_alloc_pair(&tail->tmem_base, kTmemCols);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(&tail->tmem_base, kTmemCols);
-      tmem_relinquish();
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) {
+// The work of a run, by all threads of the CTA: token tiles of the experts whose mark is `wide`, and the
+// CTA's first items.
+template <int kForm>
+__device__ __forceinline__ void build_work(const Params& p, SmemTail* tail, int wide, int rank, int w_first, int w_stride) {
+  using C = Cfg<kForm>;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
     // token tiles per expert, exclusive prefix sums: every lane takes a contiguous span of experts
     const int per = (p.E + 31) >> 5;
     const int e0 = min(p.E, lane * per), e1 = min(p.E, e0 + per);
-    int n = 0, widest = 0;
+    auto tiles = [&](int e) {
+      return tail->wide[e] == wide ? (tail->offs[e + 1] - tail->offs[e] + C::kMaxTok - 1) / C::kMaxTok : 0;
+    };
+    int n = 0, widest = 0, marked = 0;
     for (int e = e0; e < e1; ++e) {
-      const int cnt = tail->offs[e + 1] - tail->offs[e], me = (cnt + C::kMaxTok - 1) / C::kMaxTok;
+      const int me = tiles(e);
       n += me;
-      if (me > 0) widest = max(widest, (cnt + me - 1) / me);
+      marked |= tail->wide[e];
+      if (me > 0) widest = max(widest, (tail->offs[e + 1] - tail->offs[e] + me - 1) / me);
     }
     widest = __reduce_max_sync(0xffffffffu, widest);
-    if (lane == 0) tail->max_cols = max((widest + C::kColStep - 1) & ~(C::kColStep - 1), C::kColStep);
+    marked = __reduce_max_sync(0xffffffffu, marked);
+    if (lane == 0) {
+      tail->max_cols = max((widest + C::kColStep - 1) & ~(C::kColStep - 1), C::kColStep);
+      tail->any_wide = marked;
+    }
     int incl = n;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -361,22 +345,29 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
     int at = incl - n;
     for (int e = e0; e < e1; ++e) {
       tail->tile_base[e] = at;
-      at += (tail->offs[e + 1] - tail->offs[e] + C::kMaxTok - 1) / C::kMaxTok;
+      at += tiles(e);
     }
     if (lane == 31) tail->tile_base[p.E] = incl;
   }
   __syncthreads();
-  const int total_work = tail->tile_base[p.E] * p.n_tiles;
-  const int w_first = kPair ? static_cast<int>(blockIdx.x) >> 1 : static_cast<int>(blockIdx.x);
-  const int w_stride = kPair ? static_cast<int>(gridDim.x) >> 1 : static_cast<int>(gridDim.x);
-  if (static_cast<int>(threadIdx.x) < kMaxList && w_first + static_cast<int>(threadIdx.x) * w_stride < total_work) {
-    const Work c = decode_work<kForm, kTo>(w_first + static_cast<int>(threadIdx.x) * w_stride, p, tail, rank);
-    tail->list[threadIdx.x] = make_int4(c.e | (c.wide ? kWideBit : 0), c.nt, c.row0, c.nrows);
+  const int w = w_first + static_cast<int>(threadIdx.x) * w_stride;
+  if (static_cast<int>(threadIdx.x) < kMaxList && w < tail->tile_base[p.E] * p.n_tiles) {
+    const Work c = decode_work<kForm>(w, p, tail, rank);
+    tail->list[threadIdx.x] = make_int4(c.e, c.nt, c.row0, c.nrows);
   }
   __syncthreads();
-  if (kPair) cluster_sync_all();   // both CTAs' barriers are initialised before anyone signals them
-  tc_fence_after();
+}
 
+// All roles over the CTA's items of a run
+template <int EPI, int kForm, int kTo>
+__device__ __forceinline__ void run_items(const CUtensorMap& tmX64, const CUtensorMap& tmX32, const CUtensorMap& tmX16,
+                                          const CUtensorMap& tmW, const Params& p, SmemTail* tail, Bars* bars,
+                                          uint8_t* sTok, uint8_t* sRaw, int rank, int w_first, int w_stride) {
+  using C = Cfg<kForm>;
+  constexpr bool kPair = C::kPair;
+  constexpr bool kGated = EPI == EPI_FC1_GATED;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int total_work = tail->tile_base[p.E] * p.n_tiles;
   const uint32_t tmem_base = tail->tmem_base;
   volatile int* abort_flag = &tail->abort_flag;
   // a k-block of the widest tile's token rows (of this CTA's share), k-blocks per stage, stages
@@ -395,7 +386,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       uint32_t rphase = 0;
       bool ok = true;
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
+        const Work c = get_work<kForm>(it, w, p, tail, rank);
         const int nt = min(c.nt, p.n_row_tiles - 1);        // half-empty last pair: load the other half again
         const int r0 = p.sub0_base + nt * p.n_step;
         int r1 = p.sub1_base + nt * p.n_step;
@@ -407,7 +398,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
         const size_t sf_group = static_cast<size_t>(p.atoms_k) * 512;
         const int y0 = c.e * p.w_rows + r0, y1 = c.e * p.w_rows + r1;
         for (int kb = 0; kb < p.k_blocks; kb += kKBlocksPerRaw) {
-          if (!mbar_wait_bounded(&tail->rempty[rs], rphase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
+          if (!mbar_wait_bounded(&bars->rempty[rs], rphase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
             ok = false;
             break;
           }
@@ -415,7 +406,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
           uint8_t* dst = sRaw + rs * kSmemRaw;
           uint8_t* dst_sf = dst + kSmemCodes;
           const uint8_t* src_sf = sf_e + static_cast<size_t>(kb) * 512;
-          uint64_t* bar = &tail->rfull[rs];
+          uint64_t* bar = &bars->rfull[rs];
           mbar_expect_tx(bar, kSmemCodes + n_atoms * atom_bytes);
           tma_load_2d(dst, &tmW, bar, kb * 32, y0);
           tma_load_2d(dst + kSmemCodes / 2, &tmW, bar, kb * 32, y1);
@@ -437,36 +428,36 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
     // ------------------------------ token rows (pair: this CTA's half of the columns) ------------
     // a box of 64 or 32 rows and one of 16 (either may be missing) of each k-block of a stage
     if (elect_one()) {
-      for (int i = 0; i < 3; ++i) tma_prefetch_desc(&tmX.m[0][i]);
+      tma_prefetch_desc(&tmX64);
+      tma_prefetch_desc(&tmX32);
+      tma_prefetch_desc(&tmX16);
       int ts = 0;
       uint32_t tphase = 0;
       bool ok = true;
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
+        const Work c = get_work<kForm>(it, w, p, tail, rank);
         const int rows = kPair ? c.cols >> 1 : c.cols;       // 16, 32, 48, 64 or 80
         const int big = rows >= 64 ? 64 : (rows & 32);
-        const CUtensorMap* maps = tmX.m[c.wide ? 1 : 0];
-        const CUtensorMap* tm = big == 64 ? maps : maps + 1;
-        const CUtensorMap* tm16 = maps + 2;
+        const CUtensorMap* tm = big == 64 ? &tmX64 : &tmX32;
         const int y = c.row0 + (kPair ? rank * rows : 0);
         for (int kb = 0; kb < p.k_blocks; kb += tok_kbs) {
-          if (!mbar_wait_bounded(&tail->tempty[ts], tphase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
+          if (!mbar_wait_bounded(&bars->tempty[ts], tphase ^ 1, abort_flag, p.status, WAIT_SMEM_EMPTY)) {
             ok = false;
             break;
           }
           const int nk = min(tok_kbs, p.k_blocks - kb);
-          if (rank == 0) mbar_expect_tx(&tail->tfull[ts], static_cast<uint32_t>(c.cols * 128 * nk));
-          const uint32_t bar = kPair ? map_to_cta(smem_u32(&tail->tfull[ts]), 0) : 0u;
+          if (rank == 0) mbar_expect_tx(&bars->tfull[ts], static_cast<uint32_t>(c.cols * 128 * nk));
+          const uint32_t bar = kPair ? map_to_cta(smem_u32(&bars->tfull[ts]), 0) : 0u;
           for (int kq = 0; kq < nk; ++kq) {
             const int x = (kb + kq) * kKPerBlock;
             uint8_t* dst = sTok + (tok_kbs * ts + kq) * tok_kb_bytes;
             if (big != 0) {
               if (kPair) tma_load_2d_pair(dst, tm, bar, x, y);
-              else tma_load_2d(dst, tm, &tail->tfull[ts], x, y);
+              else tma_load_2d(dst, tm, &bars->tfull[ts], x, y);
             }
             if (rows != big) {
-              if (kPair) tma_load_2d_pair(dst + big * 128, tm16, bar, x, y + big);
-              else tma_load_2d(dst + big * 128, tm16, &tail->tfull[ts], x, y + big);
+              if (kPair) tma_load_2d_pair(dst + big * 128, &tmX16, bar, x, y + big);
+              else tma_load_2d(dst + big * 128, &tmX16, &bars->tfull[ts], x, y + big);
             }
           }
           if (++ts == tok_stages) {
@@ -488,9 +479,9 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       bool ok = true;
       const uint64_t bdesc0 = make_desc_sw128(smem_u32(sTok));
       for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-        const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
-        const uint32_t idesc = make_idesc_16bit(kPair ? 256 : 128, c.cols, kTo != TO_F16 || c.wide);
-        if (!mbar_wait_bounded(&tail->acc_empty[buf], acc_phase[buf] ^ 1, abort_flag, p.status, WAIT_TMEM_EMPTY)) {
+        const Work c = get_work<kForm>(it, w, p, tail, rank);
+        const uint32_t idesc = make_idesc_16bit(kPair ? 256 : 128, c.cols, kTo != TO_F16);
+        if (!mbar_wait_bounded(&bars->acc_empty[buf], acc_phase[buf] ^ 1, abort_flag, p.status, WAIT_TMEM_EMPTY)) {
           ok = false;
           break;
         }
@@ -501,8 +492,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
           constexpr int kU = decltype(units)::value;
           for (int kb = 0; kb < p.k_blocks; kb += kU) {
             const bool first_of_a = kU == C::kStageKb || kb % C::kStageKb == 0;
-            if ((first_of_a && !mbar_wait_bounded(&tail->afull[as], aphase, abort_flag, p.status, WAIT_CONVERT)) ||
-                !mbar_wait_bounded(&tail->tfull[ts], tphase, abort_flag, p.status, WAIT_SMEM_FULL)) {
+            if ((first_of_a && !mbar_wait_bounded(&bars->afull[as], aphase, abort_flag, p.status, WAIT_CONVERT)) ||
+                !mbar_wait_bounded(&bars->tfull[ts], tphase, abort_flag, p.status, WAIT_SMEM_FULL)) {
               ok = false;
               break;
             }
@@ -524,15 +515,15 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
                 bdesc += static_cast<uint32_t>(tok_kb_bytes >> 4);
               }
             }
-            if (kPair) tc_commit_pair_both(&tail->tempty[ts]);
-            else tc_commit(&tail->tempty[ts]);
+            if (kPair) tc_commit_pair_both(&bars->tempty[ts]);
+            else tc_commit(&bars->tempty[ts]);
             if (++ts == tok_stages) {
               ts = 0;
               tphase ^= 1;
             }
             if (kU == C::kStageKb || (kb + kU) % C::kStageKb == 0 || kb + kU >= p.k_blocks) {
-              if (kPair) tc_commit_pair_both(&tail->aempty[as]);
-              else tc_commit(&tail->aempty[as]);
+              if (kPair) tc_commit_pair_both(&bars->aempty[as]);
+              else tc_commit(&bars->aempty[as]);
               if (++as == C::kRing) {
                 as = 0;
                 aphase ^= 1;
@@ -543,8 +534,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
         if (tok_kbs == 4) main_loop(std::integral_constant<int, C::kStageKb>{});
         else main_loop(std::integral_constant<int, 2>{});
         if (ok) {
-          if (kPair) tc_commit_pair_both(&tail->acc_full[buf]);
-          else tc_commit(&tail->acc_full[buf]);
+          if (kPair) tc_commit_pair_both(&bars->acc_full[buf]);
+          else tc_commit(&bars->acc_full[buf]);
         }
         acc_phase[buf] ^= 1;
         buf ^= 1;
@@ -556,13 +547,13 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
     // this lane's weight row inside the staged 128: sub-tile 0 = rows 0..63, sub-tile 1 = 64..127
     const int row = kGated ? 16 * sub + (lane & 15) + 64 * (lane >> 4) : 32 * sub + lane;
     const uint32_t a_lane = tmem_base + C::kRingCol + (static_cast<uint32_t>(sub * 32) << 16);
-    const uint32_t afull0 = kPair ? map_to_cta(smem_u32(&tail->afull[0]), 0) : 0u;
+    const uint32_t afull0 = kPair ? map_to_cta(smem_u32(&bars->afull[0]), 0) : 0u;
     const uint32_t chunk_xor = static_cast<uint32_t>(row & 7) << 4;
     const int n_raw = (p.k_blocks + kKBlocksPerRaw - 1) / kKBlocksPerRaw, n_stages = (p.k_blocks + C::kStageKb - 1) / C::kStageKb;
     uint32_t raw0 = 0, stage0 = 0;   // raw stages and MMA stages before this tile
     bool ok = true;
     for (int w = w_first, it = 0; ok && w < total_work; w += w_stride, ++it) {
-      const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
+      const Work c = get_work<kForm>(it, w, p, tail, rank);
       const int nt = min(c.nt, p.n_row_tiles - 1);
       const int r0 = p.sub0_base + nt * p.n_step;
       int r1 = p.sub1_base + nt * p.n_step;
@@ -572,93 +563,88 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       const int slot = (row >> 6) * 2 + (wrow >> 7) - (first >> 7);
       const uint32_t sf_off = kSmemCodes + min(slot, 3) * 2048 + (wrow & 31) * 16 + ((wrow >> 5) & 3) * 4;
       // the two groups take the raw stages in turn
-      auto convert = [&](auto as_bf16) {
-        constexpr bool kBf16 = decltype(as_bf16)::value;     // TO_F16: re-encode for an expert marked `wide`
-        for (int r = (group + raw0) & 1; r < n_raw; r += kConvGroups) {
-          const uint32_t rs = (raw0 + r) % C::kRawStages, rphase = ((raw0 + r) / C::kRawStages) & 1u;
-          if (!mbar_wait_bounded(&tail->rfull[rs], rphase, abort_flag, p.status, WAIT_CONVERT)) {
+      for (int r = (group + raw0) & 1; r < n_raw; r += kConvGroups) {
+        const uint32_t rs = (raw0 + r) % C::kRawStages, rphase = ((raw0 + r) / C::kRawStages) & 1u;
+        if (!mbar_wait_bounded(&bars->rfull[rs], rphase, abort_flag, p.status, WAIT_CONVERT)) {
+          ok = false;
+          break;
+        }
+        const uint8_t* raw = sRaw + rs * kSmemRaw;
+        const uint8_t* codes = raw + row * 128;
+        const int nk = min(kKBlocksPerRaw, p.k_blocks - r * kKBlocksPerRaw);
+#pragma unroll
+        for (int q = 0; q < kKBlocksPerRaw / C::kStageKb; ++q) {   // the one or two MMA stages of the raw stage
+          if (C::kStageKb * q >= nk) break;
+          const uint32_t si = stage0 + (kKBlocksPerRaw / C::kStageKb) * r + q;
+          const uint32_t as = si % C::kRing, aphase = (si / C::kRing) & 1u;
+          if (!mbar_wait_bounded(&bars->aempty[as], aphase ^ 1, abort_flag, p.status, WAIT_CONVERT)) {
             ok = false;
             break;
           }
-          const uint8_t* raw = sRaw + rs * kSmemRaw;
-          const uint8_t* codes = raw + row * 128;
-          const int nk = min(kKBlocksPerRaw, p.k_blocks - r * kKBlocksPerRaw);
+          tc_fence_after();
+          const uint32_t a_t = a_lane + as * C::kStageCols;
+          // the k-blocks of the stage (missing ones: unread values); the next one's codes are fetched
+          // ahead of this one's stores
+          const int k0 = C::kStageKb * q;
+          uint4 nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * k0 << 4) ^ chunk_xor));
+          uint4 nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * k0 + 1) << 4) ^ chunk_xor));
+          uint32_t nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + k0 * 512);
 #pragma unroll
-          for (int q = 0; q < kKBlocksPerRaw / C::kStageKb; ++q) {   // the one or two MMA stages of the raw stage
-            if (C::kStageKb * q >= nk) break;
-            const uint32_t si = stage0 + (kKBlocksPerRaw / C::kStageKb) * r + q;
-            const uint32_t as = si % C::kRing, aphase = (si / C::kRing) & 1u;
-            if (!mbar_wait_bounded(&tail->aempty[as], aphase ^ 1, abort_flag, p.status, WAIT_CONVERT)) {
-              ok = false;
-              break;
+          for (int hk = 0; hk < C::kStageKb; ++hk) {
+            const uint4 cw[2] = {nx0, nx1};
+            const uint32_t sfw = nsf;
+            if (hk + 1 < C::kStageKb) {
+              nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * (k0 + hk + 1) << 4) ^ chunk_xor));
+              nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * (k0 + hk + 1) + 1) << 4) ^ chunk_xor));
+              nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + (k0 + hk + 1) * 512);
             }
-            tc_fence_after();
-            const uint32_t a_t = a_lane + as * C::kStageCols;
-            // the k-blocks of the stage (missing ones: unread values); the next one's codes are fetched
-            // ahead of this one's stores
-            const int k0 = C::kStageKb * q;
-            uint4 nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * k0 << 4) ^ chunk_xor));
-            uint4 nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * k0 + 1) << 4) ^ chunk_xor));
-            uint32_t nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + k0 * 512);
+            uint32_t s01 = 0, s23 = 0;
+            if (kTo != TO_BF16_E8M0) cvt_e4m3x4_f16(sfw, s01, s23);
 #pragma unroll
-            for (int hk = 0; hk < C::kStageKb; ++hk) {
-              const uint4 cw[2] = {nx0, nx1};
-              const uint32_t sfw = nsf;
-              if (hk + 1 < C::kStageKb) {
-                nx0 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>(2 * (k0 + hk + 1) << 4) ^ chunk_xor));
-                nx1 = *reinterpret_cast<const uint4*>(codes + (static_cast<uint32_t>((2 * (k0 + hk + 1) + 1) << 4) ^ chunk_xor));
-                nsf = *reinterpret_cast<const uint32_t*>(raw + sf_off + (k0 + hk + 1) * 512);
-              }
-              uint32_t s01 = 0, s23 = 0;
-              if (kTo == TO_F16) cvt_e4m3x4_f16(sfw, s01, s23);
+            for (int h = 0; h < 2; ++h) {                    // 32 codes -> 16 TMEM columns
+              const uint4 v = cw[h];
+              const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+              uint32_t out[16];
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {                    // 32 codes -> 16 TMEM columns
-                const uint4 v = cw[h];
-                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-                uint32_t out[16];
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {                  // 16 values per scale
-                  uint32_t o0[4], o1[4];
-                  if (kTo == TO_F16) {
-                    const uint32_t sc = __byte_perm(h == 0 ? s01 : s23, 0u, b == 0 ? 0x1010u : 0x3232u);
-                    cvt_e2m1x8_scaled_f16(words[2 * b], sc, o0);
-                    cvt_e2m1x8_scaled_f16(words[2 * b + 1], sc, o1);
-                  } else {
-                    const uint32_t sb = (sfw >> (16 * h + 8 * b)) & 0xffu;
-                    // E8M0: 2^(b-127) is the f32 with exponent field b (b = 0: the subnormal 2^-127)
-                    const __nv_bfloat16 s1 = __float2bfloat16_rn(__uint_as_float(sb != 0u ? sb << 23 : 0x00400000u));
-                    const __nv_bfloat162 sc = __halves2bfloat162(s1, s1);
-                    cvt_e2m1x8_bf16(words[2 * b], sc, o0);
-                    cvt_e2m1x8_bf16(words[2 * b + 1], sc, o1);
-                  }
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) {
-                    out[8 * b + i] = o0[i];
-                    out[8 * b + 4 + i] = o1[i];
-                  }
+              for (int b = 0; b < 2; ++b) {                  // 16 values per scale
+                uint32_t o0[4], o1[4];
+                if (kTo != TO_BF16_E8M0) {
+                  const uint32_t sc = __byte_perm(h == 0 ? s01 : s23, 0u, b == 0 ? 0x1010u : 0x3232u);
+                  cvt_e2m1x8_scaled_f16(words[2 * b], sc, o0);
+                  cvt_e2m1x8_scaled_f16(words[2 * b + 1], sc, o1);
+                } else {
+                  const uint32_t sb = (sfw >> (16 * h + 8 * b)) & 0xffu;
+                  // E8M0: 2^(b-127) is the f32 with exponent field b (b = 0: the subnormal 2^-127)
+                  const __nv_bfloat16 s1 = __float2bfloat16_rn(__uint_as_float(sb != 0u ? sb << 23 : 0x00400000u));
+                  const __nv_bfloat162 sc = __halves2bfloat162(s1, s1);
+                  cvt_e2m1x8_bf16(words[2 * b], sc, o0);
+                  cvt_e2m1x8_bf16(words[2 * b + 1], sc, o1);
                 }
-                if (kBf16) {
 #pragma unroll
-                  for (int i = 0; i < 16; ++i) out[i] = f16x2_to_bf16x2(out[i]);
+                for (int i = 0; i < 4; ++i) {
+                  out[8 * b + i] = o0[i];
+                  out[8 * b + 4 + i] = o1[i];
                 }
-                tc_st_32x32b_x16(a_t + 32 * hk + 16 * h, out);
               }
-            }
-            tc_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              if (kPair) mbar_arrive_cluster(afull0 + as * static_cast<uint32_t>(sizeof(uint64_t)));
-              else mbar_arrive(&tail->afull[as]);
+              if (kTo == TO_BF16_E4M3) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) out[i] = f16x2_to_bf16x2(out[i]);
+              }
+              tc_st_32x32b_x16(a_t + 32 * hk + 16 * h, out);
             }
           }
-          // this warp has read all it needs of the stage's codes and atoms
+          tc_wait_st();
+          tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&tail->rempty[rs]);
+          if (lane == 0) {
+            if (kPair) mbar_arrive_cluster(afull0 + as * static_cast<uint32_t>(sizeof(uint64_t)));
+            else mbar_arrive(&bars->afull[as]);
+          }
         }
-      };
-      if (kTo == TO_F16 && c.wide) convert(std::true_type{});
-      else convert(std::false_type{});
+        // this warp has read all it needs of the stage's codes and atoms
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->rempty[rs]);
+      }
       raw0 += n_raw;
       stage0 += n_stages;
     }
@@ -666,11 +652,11 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
     // ------------------------------ epilogue (both CTAs of a pair) --------------------------------
     // the two warps of a sub-partition take every other 32 token columns (FC1) / 16 (FC2)
     const int sub = warp & 3, half = (warp - 4 - kConvWarps) >> 2;
-    const uint32_t release0 = kPair ? map_to_cta(smem_u32(&tail->acc_empty[0]), 0) : 0u;
+    const uint32_t release0 = kPair ? map_to_cta(smem_u32(&bars->acc_empty[0]), 0) : 0u;
     uint32_t acc_phase[2] = {0, 0};
     int buf = 0;
     for (int w = w_first, it = 0; w < total_work; w += w_stride, ++it) {
-      const Work c = get_work<kForm, kTo>(it, w, p, tail, rank);
+      const Work c = get_work<kForm>(it, w, p, tail, rank);
       const float alpha = p.alphas[c.e];
       // lane l holds the factors of token t + l of the warp's next 32 (FC2: 16) columns; the first are
       // fetched before the accumulator is waited for
@@ -678,9 +664,8 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       auto row_of = [&](int t) {
         return c.row0 + min(t + (EPI == EPI_FC2 ? (lane & 15) : lane), c.nrows - 1);
       };
-      auto inv_of = [&](int t) { return c.wide ? 1.0f : p.row_inv[row_of(t)]; };
-      float inv_next = kTo == TO_F16 ? inv_of(t_first) : 1.0f;
-      if (!mbar_wait_idle(&tail->acc_full[buf], acc_phase[buf], abort_flag, p.status, WAIT_TMEM_FULL)) break;
+            float inv_next = kTo == TO_F16 ? p.row_inv[row_of(t_first)] : 1.0f;
+      if (!mbar_wait_idle(&bars->acc_full[buf], acc_phase[buf], abort_flag, p.status, WAIT_TMEM_FULL)) break;
       acc_phase[buf] ^= 1;
       tc_fence_after();
       const uint32_t t_lane = tmem_base + buf * C::kMaxTok + (static_cast<uint32_t>(sub * 32) << 16);
@@ -693,7 +678,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
           tc_ld_32x32b_x16(t_lane + ch, r);
           tc_wait_ld();
           const float inv_l = inv_next;
-          if (kTo == TO_F16 && ch + 32 < c.cols) inv_next = inv_of(ch + 32);
+          if (kTo == TO_F16 && ch + 32 < c.cols) inv_next = p.row_inv[row_of(ch + 32)];
           float* o = p.out_f32 + static_cast<size_t>(c.row0 + ch) * p.out_cols + col;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -705,7 +690,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       } else {
         for (int t0 = 32 * half; t0 < c.cols; t0 += 64) {
           const float inv_l = inv_next;
-          if (kTo == TO_F16 && t0 + 64 < c.cols) inv_next = inv_of(t0 + 64);
+          if (kTo == TO_F16 && t0 + 64 < c.cols) inv_next = p.row_inv[row_of(t0 + 64)];
           const float al_l = p.route_weights != nullptr
                                  ? __fmul_rn(alpha, p.route_weights[p.sorted_route_ids[row_of(t0)]]) : alpha;
 #pragma unroll
@@ -786,10 +771,79 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
       __syncwarp();
       if (lane == 0) {
         if (kPair) mbar_arrive_cluster(release0 + static_cast<uint32_t>(buf * sizeof(uint64_t)));
-        else mbar_arrive(&tail->acc_empty[buf]);
+        else mbar_arrive(&bars->acc_empty[buf]);
       }
       buf ^= 1;
     }
+  }
+}
+
+// The run of the marked experts, on BF16 operands.  The other run has ended, here and in the other CTA of a pair; its
+// barriers may still be signalled by commits that nobody waits for, so this one has a set of its own.
+template <int EPI, int kForm>
+__device__ __noinline__ void run_wide_items(const CUtensorMap& tmB64, const CUtensorMap& tmB32, const CUtensorMap& tmB16,
+                                            const CUtensorMap& tmW, const Params& p, SmemTail* tail, uint8_t* sTok,
+                                            uint8_t* sRaw, int rank, int w_first, int w_stride) {
+  if (threadIdx.x == 0) init_bars<kForm>(&tail->bars[1]);
+  tc_fence_before();
+  __syncthreads();
+  build_work<kForm>(p, tail, 1, rank, w_first, w_stride);
+  if (Cfg<kForm>::kPair) cluster_sync_all();
+  tc_fence_after();
+  run_items<EPI, kForm, TO_BF16_E4M3>(tmB64, tmB32, tmB16, tmW, p, tail, &tail->bars[1], sTok, sRaw, rank, w_first, w_stride);
+}
+
+// tmX*: the token rows as kTo says, boxes of 64, 32 and 16 rows; tmB*: TO_F16: the same rows as BF16
+template <int EPI, int kForm, int kTo>
+__global__ void __launch_bounds__(kThreads, 1)
+grouped_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmX64, const __grid_constant__ CUtensorMap tmX32,
+                          const __grid_constant__ CUtensorMap tmX16, const __grid_constant__ CUtensorMap tmB64,
+                          const __grid_constant__ CUtensorMap tmB32, const __grid_constant__ CUtensorMap tmB16,
+                          const __grid_constant__ CUtensorMap tmW, const __grid_constant__ Params p) {
+  using C = Cfg<kForm>;
+  constexpr bool kPair = C::kPair;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* sTok = smem;
+  uint8_t* sRaw = sTok + C::kSmemTok;
+  SmemTail* tail = reinterpret_cast<SmemTail*>(sRaw + C::kRawStages * kSmemRaw);
+  const int warp = threadIdx.x >> 5;
+  const int rank = kPair ? static_cast<int>(cluster_ctarank()) : 0;
+
+  if (threadIdx.x == 0) {
+    tail->abort_flag = 0;
+    init_bars<kForm>(&tail->bars[0]);
+  }
+  for (int i = threadIdx.x; i <= p.E; i += kThreads) {
+    tail->offs[i] = p.expert_offsets[i];
+    if (i < p.E) tail->wide[i] = kTo == TO_F16 && p.wide[i] != 0;
+  }
+  if (warp == 1) {
+    if (kPair) {
+      tmem_alloc_pair(&tail->tmem_base, kTmemCols);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&tail->tmem_base, kTmemCols);
+      tmem_relinquish();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  const int w_first = kPair ? static_cast<int>(blockIdx.x) >> 1 : static_cast<int>(blockIdx.x);
+  const int w_stride = kPair ? static_cast<int>(gridDim.x) >> 1 : static_cast<int>(gridDim.x);
+  build_work<kForm>(p, tail, 0, rank, w_first, w_stride);
+  if (kPair) cluster_sync_all();   // both CTAs' barriers are initialised before anyone signals them
+  tc_fence_after();
+  run_items<EPI, kForm, kTo>(tmX64, tmX32, tmX16, tmW, p, tail, &tail->bars[0], sTok, sRaw, rank, w_first, w_stride);
+
+  if (kTo == TO_F16 && tail->any_wide != 0) {
+    // the marked experts' items go round on from where the others ended: CTAs short of an item take one first
+    const int first = (w_first + w_stride - tail->tile_base[p.E] * p.n_tiles % w_stride) % w_stride;
+    tc_fence_before();
+    __syncthreads();
+    if (kPair) cluster_sync_all();
+    run_wide_items<EPI, kForm>(tmB64, tmB32, tmB16, tmW, p, tail, sTok, sRaw, rank, first, w_stride);
   }
 
   // ------------------------------ teardown ------------------------------------
@@ -797,6 +851,7 @@ grouped_gemm_w4a16_kernel(const __grid_constant__ TokenMaps tmX, const __grid_co
   __syncthreads();
   if (kPair) cluster_sync_all();   // nobody signals the other CTA's shared memory after this
   if (warp == 1) {
+    const uint32_t tmem_base = tail->tmem_base;
     tc_fence_after();
     if (kPair) tmem_dealloc_pair(tmem_base, kTmemCols);
     else tmem_dealloc(tmem_base, kTmemCols);
@@ -861,28 +916,56 @@ __global__ void __launch_bounds__(256) permute_rows_bf16_kernel(
 
 // The same, and the rows once more as FP16 (rows_bf16 and sorted_route_ids null: rows that lie in sorted order
 // already, FC2's, as FP16 only), each multiplied by the power of two that puts its largest finite magnitude
-// into [2^14, 2^15); row_inv[pos] takes the inverse.  BF16 has 8 significant bits: every value down to 2^-31
+// into [2^15, 2^16); row_inv[pos] takes the inverse.  BF16 has 8 significant bits: every value down to 2^-32
 // of the row's largest binade is carried over exactly.  A row with smaller ones marks its expert `wide`
 // (a mark too many is still right: such an expert's GEMMs run on the BF16 rows, at a lower rate; the sort clears
 // the marks).  Infinities and NaNs stay what they are.
+//
+// Bound by its bytes for many rows (FC1, 32768 of 4096: 125 us for 268 MB read and 537 MB written, about 70 us
+// without the BF16 copy), by the latency of one row's two passes for few: there the eight warps of a CTA share a
+// row (512 rows of 14336: 34 -> 8 us).
+template <int kWarps, bool kCopy>
 __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* __restrict__ expert_offsets,
     int E, const int32_t* __restrict__ sorted_route_ids, int num_topk, int K,
     __nv_bfloat16* __restrict__ rows_bf16, __half* __restrict__ out, float* __restrict__ row_inv,
     int32_t* __restrict__ wide) {
+  __shared__ uint32_t part_most[8];
+  __shared__ int part_least[8];
   const int total = expert_offsets[E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nvec = K >> 3;
-  for (int pos = blockIdx.x * 8 + warp; pos < total; pos += gridDim.x * 8) {
+  const int nvec = K >> 3, first = lane + 32 * (warp % kWarps);
+  constexpr int kRows = 8 / kWarps, kStep = 32 * kWarps;
+  // over the warps of the row (all threads of the CTA in step, if they share one)
+  auto row_max = [&](uint32_t v) -> uint32_t {
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (kWarps == 1) return v;
+    __syncthreads();
+    if (lane == 0) part_most[warp] = v;
+    __syncthreads();
+    for (int i = 0; i < kWarps; ++i) v = max(v, part_most[i]);
+    return v;
+  };
+  auto row_min = [&](int v) -> int {
+    v = __reduce_min_sync(0xffffffffu, v);
+    if (kWarps == 1) return v;
+    __syncthreads();
+    if (lane == 0) part_least[warp] = v;
+    __syncthreads();
+    for (int i = 0; i < kWarps; ++i) v = min(v, part_least[i]);
+    return v;
+  };
+  for (int pos = blockIdx.x * kRows + warp / kWarps; pos < total; pos += gridDim.x * kRows) {
     const int tkn = sorted_route_ids != nullptr ? sorted_route_ids[pos] / num_topk : pos;
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(tkn) * x_row_stride);
-    uint4* copy = rows_bf16 != nullptr ? reinterpret_cast<uint4*>(rows_bf16 + static_cast<size_t>(pos) * K) : nullptr;
+    uint4* copy = kCopy ? reinterpret_cast<uint4*>(rows_bf16 + static_cast<size_t>(pos) * K) : nullptr;
     __nv_bfloat162 m2 = __float2bfloat162_rn(0.f);
     // smallest nonzero magnitude: + 0x7fff takes 0 to the largest signed 16-bit value and keeps the others in order
     uint32_t least2 = 0x7fff7fffu;
-    for (int j = lane; j < nvec; j += 32) {
+#pragma unroll 4
+    for (int j = first; j < nvec; j += kStep) {
       const uint4 v = __ldg(src + j);
-      if (copy != nullptr) copy[j] = v;
+      if (kCopy) copy[j] = v;
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -891,11 +974,11 @@ __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
       }
     }
     // BF16 magnitudes order like their bits
-    uint32_t m = __reduce_max_sync(0xffffffffu, static_cast<uint32_t>(max(__bfloat16_as_ushort(__low2bfloat16(m2)),
-                                                                          __bfloat16_as_ushort(__high2bfloat16(m2)))));
+    uint32_t m = row_max(static_cast<uint32_t>(max(__bfloat16_as_ushort(__low2bfloat16(m2)),
+                                                   __bfloat16_as_ushort(__high2bfloat16(m2)))));
     if (m >= 0x7f80u) {            // an infinity: once more over the finite values
       m = 0;
-      for (int j = lane; j < nvec; j += 32) {
+      for (int j = first; j < nvec; j += kStep) {
         const uint4 v = __ldg(src + j);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -905,15 +988,15 @@ __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
           if (hi < 0x7f80u) m = max(m, hi);
         }
       }
-      m = __reduce_max_sync(0xffffffffu, m);
+      m = row_max(m);
     }
-    // exponent field e of the largest: x 2^(141 - e), the factor kept a normal float either way
-    const int sh = min(141 - max(static_cast<int>(m >> 7), 1), 126);
+    // exponent field e of the largest: x 2^(142 - e), the factor kept a normal float either way
+    const int sh = min(142 - max(static_cast<int>(m >> 7), 1), 126);
     const float scale = __uint_as_float(static_cast<uint32_t>(127 + sh) << 23);
     // the last bit of a value with exponent field f is 2^(f - 134 + sh) of the FP16 row, whose last is 2^-24
-    const int least = __reduce_min_sync(0xffffffffu, min(static_cast<int>(static_cast<int16_t>(least2 & 0xffffu)),
-                                                         static_cast<int>(least2) >> 16)) + 0x8001;
-    if (lane == 0) {
+    const int least = row_min(min(static_cast<int>(static_cast<int16_t>(least2 & 0xffffu)),
+                                  static_cast<int>(least2) >> 16)) + 0x8001;
+    if (first == 0) {
       row_inv[pos] = __uint_as_float(static_cast<uint32_t>(127 - sh) << 23);
       if (max(least >> 7, 1) + sh < 110) {
         int lo = 0, hi = E - 1;      // the expert of the row: the last whose first row is not behind it
@@ -925,7 +1008,8 @@ __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
       }
     }
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(pos) * K);
-    for (int j = lane; j < nvec; j += 32) {
+#pragma unroll 4
+    for (int j = first; j < nvec; j += kStep) {
       const uint4 v = __ldg(src + j);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
       uint32_t o[4];
@@ -938,6 +1022,18 @@ __global__ void __launch_bounds__(256) permute_rows_f16_kernel(
       dst[j] = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
+}
+
+// copy: the rows as BF16 too (FC1; null for rows that lie in sorted order already)
+static int launch_rows_f16(int rows, const __nv_bfloat16* x, int64_t x_row_stride, const int32_t* expert_offsets, int E,
+                           const int32_t* sorted_route_ids, int num_topk, int K, __nv_bfloat16* copy, __half* out,
+                           float* row_inv, int32_t* wide, cudaStream_t s) {
+  constexpr int kFull = 148 * 8;                       // CTAs of 256 threads that run at once
+  auto kern = rows <= kFull ? (copy != nullptr ? permute_rows_f16_kernel<8, true> : permute_rows_f16_kernel<8, false>)
+                            : (copy != nullptr ? permute_rows_f16_kernel<1, true> : permute_rows_f16_kernel<1, false>);
+  const int grid = rows <= kFull ? rows : ((rows + 7) / 8 < kFull ? (rows + 7) / 8 : kFull);
+  kern<<<grid, 256, 0, s>>>(x, x_row_stride, expert_offsets, E, sorted_route_ids, num_topk, K, copy, out, row_inv, wide);
+  return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }
 
 // 2-D bf16 matrix [rows][cols], box = box_rows x 64 elements (128 bytes), 128-byte swizzle
@@ -973,7 +1069,7 @@ static int make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t cols, uin
 }
 
 template <int EPI, int kForm, int kTo>
-static int launch(const TokenMaps& tmX, const CUtensorMap& tmW, const Params& p, int ctas, cudaStream_t s) {
+static int launch(const CUtensorMap (&tmX)[6], const CUtensorMap& tmW, const Params& p, int ctas, cudaStream_t s) {
   constexpr bool kPair = Cfg<kForm>::kPair;
   auto kern = grouped_gemm_w4a16_kernel<EPI, kForm, kTo>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<kForm>()) != cudaSuccess)
@@ -996,7 +1092,7 @@ static int launch(const TokenMaps& tmX, const CUtensorMap& tmW, const Params& p,
     if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) return B200MOE_ECUDA;
     if (2 * clusters < static_cast<int>(cfg.gridDim.x)) cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
   }
-  return cudaLaunchKernelEx(&cfg, kern, tmX, tmW, p) == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
+  return cudaLaunchKernelEx(&cfg, kern, tmX[0], tmX[1], tmX[2], tmX[3], tmX[4], tmX[5], tmW, p) == cudaSuccess ? B200MOE_OK : B200MOE_ECUDA;
 }
 
 // One CTA up to 18 rows per expert (finer tiles, no partner to wait for), narrow pairs to 58 (nearly every
@@ -1026,12 +1122,11 @@ static int form_for(const b200moe_gemm_args* a, int ctas) {
 template <int EPI, int kTo>
 static int launch_any(const b200moe_gemm_args* a, const void* tokens, const void* tokens_bf16, uint64_t cols,
                       const void* weights, Params& p, cudaStream_t s) {
-  TokenMaps tmX;
-  CUtensorMap tmW;
+  CUtensorMap tmX[6], tmW;      // the token rows as kTo says, then as BF16
   const uint32_t boxes[3] = {64, 32, 16};
   for (int i = 0; i < 3; ++i) {
-    int rc = make_tmap_bf16(&tmX.m[0][i], tokens, cols, a->layout->rows, boxes[i]);
-    if (rc == B200MOE_OK) rc = make_tmap_bf16(&tmX.m[1][i], tokens_bf16, cols, a->layout->rows, boxes[i]);
+    int rc = make_tmap_bf16(&tmX[i], tokens, cols, a->layout->rows, boxes[i]);
+    if (rc == B200MOE_OK) rc = make_tmap_bf16(&tmX[3 + i], tokens_bf16, cols, a->layout->rows, boxes[i]);
     if (rc != B200MOE_OK) return rc;
   }
   const int rc = make_tmap_bytes_2d(&tmW, weights, cols / 2, static_cast<uint64_t>(a->num_experts) * p.w_rows, 64);
@@ -1085,15 +1180,17 @@ int w4a16_gemm1(const b200moe_gemm_args* a, cudaStream_t stream) {
   const int32_t* offsets = reinterpret_cast<const int32_t*>(base + L.expert_offsets);
   const int32_t* routes = reinterpret_cast<const int32_t*>(base + L.sorted_route_ids);
   int32_t* wide = wide_marks(a, base);
-  if (f16)
-    permute_rows_f16_kernel<<<ggrid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes, a->num_topk, K,
-        reinterpret_cast<__nv_bfloat16*>(base + L.act_q), reinterpret_cast<__half*>(base + L.mid_sf),
-        reinterpret_cast<float*>(base + L.act_sf), wide);
-  else
+  if (f16) {
+    const int rc = launch_rows_f16(rows, static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes,
+                                   a->num_topk, K, reinterpret_cast<__nv_bfloat16*>(base + L.act_q),
+                                   reinterpret_cast<__half*>(base + L.mid_sf), reinterpret_cast<float*>(base + L.act_sf),
+                                   wide, stream);
+    if (rc != B200MOE_OK) return rc;
+  } else {
     permute_rows_bf16_kernel<<<ggrid, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(a->x), a->x_row_stride, offsets, E, routes, a->num_topk, K,
         reinterpret_cast<__nv_bfloat16*>(base + L.act_q));
+  }
   const void* tokens = base + (f16 ? L.mid_sf : L.act_q);
   Params p = {};
   fill_common(p, a, base);
@@ -1151,9 +1248,9 @@ int w4a16_gemm2(const b200moe_gemm_args* a, cudaStream_t stream) {
   const int rows = a->num_tokens * a->num_topk;
   float* row_inv = reinterpret_cast<float*>(base + L.act_sf) + L.rows;
   int32_t* wide = wide_marks(a, base) + E;
-  permute_rows_f16_kernel<<<row_grid(rows), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(base + L.mid_q), I, p.expert_offsets, E, nullptr, 1, I, nullptr,
-      reinterpret_cast<__half*>(base + L.mid_sf), row_inv, wide);
+  const int rc = launch_rows_f16(rows, reinterpret_cast<const __nv_bfloat16*>(base + L.mid_q), I, p.expert_offsets, E,
+                                 nullptr, 1, I, nullptr, reinterpret_cast<__half*>(base + L.mid_sf), row_inv, wide, stream);
+  if (rc != B200MOE_OK) return rc;
   p.row_inv = row_inv;
   p.wide = wide;
   return launch_any<EPI_FC2, TO_F16>(a, base + L.mid_sf, base + L.mid_q, I, a->w2, p, stream);

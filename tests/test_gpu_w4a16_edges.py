@@ -117,7 +117,7 @@ def _rowwise(got, ref, tol):
                                                 (140, 2, "relu2")])
 def test_rows_wider_than_fp16(tokens, experts, act):
     """Rows whose largest element lies 20 to 60 binades above the others and meets a zero weight, so that the small
-    elements are the whole sum: up to 31 binades on FP16 operands (expert 0), beyond on BF16 operands."""
+    elements are the whole sum: up to 32 binades on FP16 operands (expert 0), beyond on BF16 operands."""
     shp = _w16(tokens=tokens, experts=experts, topk=1, hidden=320, intermediate=192, activation=act)
     inp = synth.make_inputs(shp, seed=tokens)
     gap = 20 + torch.arange(tokens) * 41 // tokens
@@ -132,6 +132,24 @@ def test_rows_wider_than_fp16(tokens, experts, act):
     run = run_layer(inp, topk_ids=ids, topk_weights=torch.ones(tokens, 1))
     _, taps = oracle_layer(inp, ids, torch.ones(tokens, 1))
     _rowwise(run.fc1[:tokens], taps.fc1, 1e-4)          # fp32 sums of 320 terms in another order
+
+
+def test_one_row_wider_than_fp16_among_others():
+    """One row of one of two experts puts that expert on BF16 operands: the other rows keep their bits."""
+    shp = _w16(tokens=400, experts=2, topk=1, hidden=320, intermediate=192)
+    inp = synth.make_inputs(shp, seed=2)
+    w1 = inp.w1_fp4.clone()
+    w1[..., 0] &= 0xF0
+    x = inp.x.float().cpu()
+    ids, w = (torch.arange(400) >= 100).to(torch.int32).reshape(-1, 1), torch.ones(400, 1)
+    plain = run_layer(replace(inp, w1_fp4=w1), topk_ids=ids, topk_weights=w)
+    x[200] = 2.0 ** -36
+    x[200, 0] = 16.0
+    run = run_layer(replace(inp, x=x.to(torch.bfloat16), w1_fp4=w1), topk_ids=ids, topk_weights=w)
+    keep = [i for i in range(400) if i != 200]
+    assert torch.equal(run.fc1[keep], plain.fc1[keep]) and torch.equal(run.out_f32[keep], plain.out_f32[keep])
+    _, taps = oracle_layer(run.inp, ids, w)
+    _rowwise(run.fc1[200:201], taps.fc1[200:201], 1e-4)
 
 
 @pytest.mark.parametrize("tokens,experts", [(30, 4), (40, 2), (140, 2)])
